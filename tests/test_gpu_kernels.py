@@ -1,5 +1,6 @@
 """Numerics of every CUDA kernel against the plain PyTorch fp32 reference (needs a B200)."""
 import ctypes as C
+import math
 
 import numpy as np
 import pytest
@@ -542,3 +543,44 @@ def test_fused_sgd_takes_channels_last_and_mixed_groups():
     assert [p.grad.data_ptr() for p in own_p] == ptrs and all(float(p.grad.abs().max()) == 0 for p in own_p)
     own_opt.zero_grad()
     assert all(p.grad is None for p in own_p)
+
+
+def _exact_lamb(p, g, m, v, lr, b1, b2, eps, wd, step, clip):
+    p, g, m, v = (t.double() for t in (p, g, m, v))
+    lr, b1, b2, eps, wd = (float(np.float32(x)) for x in (lr, b1, b2, eps, wd))      # the kernel's arguments
+    g = g * clip
+    m, v = b1 * m + (1 - b1) * g, b2 * v + (1 - b2) * g * g
+    u = (m / (1 - b1 ** step)) / ((v / (1 - b2 ** step)).sqrt() + eps) + wd * p
+    pn, un = p.norm(), u.norm()
+    return p - lr * (float(pn / un) if pn > 0 and un > 0 else 1.0) * u, m, v
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_lamb_slices_and_misaligned_tensors(shift):
+    """Tensor lengths around the slice, the 16-byte group and the chunk of the LAMB kernels, with parameters and
+    gradients that start ``shift`` elements behind a 16-byte boundary, against 64 bits.  Tolerance: 32-bit sums of
+    65,537 squares and a handful of roundings per element, 1e-5 relative to the tensor's largest entry."""
+    from conef_b200.optim import FusedLAMB
+
+    sizes = [1, 3, 4, 5, 2047, 8191, 8192, 8193, 65535, 65536, 65537, 3 * 65536 + 8194]
+    gen = torch.Generator().manual_seed(5)
+    rand = lambda n: torch.randn(n, generator=gen)
+    off = lambda t: torch.cat([torch.zeros(shift), t]).to(DEV)[shift:]
+    params = [torch.nn.Parameter(off(rand(n))) for n in sizes]
+    assert all(p.data_ptr() % 16 == 4 * shift for p in params)
+    opt = FusedLAMB([{"params": params[::2], "weight_decay": 0.01}, {"params": params[1::2], "weight_decay": 0.0}], lr=1e-2)
+    start = [p.detach().clone() for p in params]
+    for p in params:
+        p.grad = off(rand(p.numel()))
+    grads = [p.grad.clone() for p in params]
+    native.reset_launch_count()
+    opt.step()
+    norm = math.sqrt(sum(float(g.double().pow(2).sum()) for g in grads))
+    group = opt.param_groups[0]
+    clip = min(1.0, group["max_grad_norm"] / norm) if group["max_grad_norm"] else 1.0
+    for k, p in enumerate(params):
+        zero = torch.zeros_like(grads[k])
+        want = _exact_lamb(start[k], grads[k], zero, zero, 1e-2, *group["betas"], group["eps"], 0.01 if k % 2 == 0 else 0.0,
+                           1, clip)
+        for got, w in zip((p.detach(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"]), want):
+            assert float((got.double() - w).abs().max()) <= 1e-5 * float(w.abs().max()), (sizes[k], k)
