@@ -953,11 +953,13 @@ extern "C" int conef_orthogonalize_packed(const ConefMat* mats, const int2* tile
 // ---------------------------------------------------------------------------
 // Corrections of the low-rank error store.
 //
-// k_corr_reduce: C = L^T Rm over the chunk's rows.  The rows come into shared memory in sub-chunks
-// with coalesced loads first: summing straight from global memory leaves one load in flight per
-// thread (the loop over rows is a chain of dependent-latency iterations) and took 70-130 us per
-// launch on a Transformer-sized bucket.
-constexpr int CR_SUB = 128;                       // rows per sub-chunk
+// k_corr_reduce: C = L^T Rm over 128 of the chunk's rows (blockIdx.y: which quarter of the 512).  The rows come
+// into shared memory with coalesced loads first: summing straight from global memory leaves one load in flight per
+// thread (the loop over rows is a chain of dependent-latency iterations) and took 70-130 us per launch on a
+// Transformer-sized bucket.  Both kernels are latency-bound: a bucket has a few dozen 512-row chunks, so a CTA per
+// chunk left five of six SMs idle; on the Transformer bucket (12 matrices,
+// rank 8) the four launches of a step took 54 + 39 us and take 19 + 26 us.
+constexpr int CR_SUB = 128;                       // rows per CTA
 __global__ void __launch_bounds__(OC_THREADS)
 k_corr_reduce(const ConefCorr* __restrict__ table, const int2* __restrict__ tiles, const float* __restrict__ L0b,
               const float* __restrict__ R0b, const float* __restrict__ L1b, const float* __restrict__ R1b,
@@ -967,8 +969,9 @@ k_corr_reduce(const ConefCorr* __restrict__ table, const int2* __restrict__ tile
   __shared__ float part[OC_THREADS / 32][256];
   const int2 t = tiles[blockIdx.x];
   const ConefCorr K = table[t.x];
-  const int row0 = t.y * OC_ROWS;
-  const int rows = min(OC_ROWS, K.rows_l - row0);
+  const int row0 = t.y * OC_ROWS + blockIdx.y * CR_SUB;
+  const int rows = min(CR_SUB, K.rows_l - row0);
+  if (rows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int term = 0; term < K.nterms; ++term) {
     const int c2 = K.c2[term], c1 = K.c1;
@@ -976,36 +979,33 @@ k_corr_reduce(const ConefCorr* __restrict__ table, const int2* __restrict__ tile
     const float* L = (term ? L1b : L0b) + K.l_off[term] + (size_t)row0 * c2;
     const float* Rm = (term ? R1b : R0b) + K.r_off[term] + (size_t)row0 * c1;
     float* c = cbuf + ((size_t)t.x * 2 + term) * GRAM_STRIDE;
-    // every warp owns a slice of each sub-chunk's rows; lanes own pairs (a, b) = (pr / c1, pr % c1)
+    // every warp owns a slice of the rows; lanes own pairs (a, b) = (pr / c1, pr % c1)
     float acc[8];                                  // pairs handled by this lane: pr = lane + 32 u (pairs <= 256)
 #pragma unroll
     for (int u = 0; u < 8; ++u) acc[u] = 0.f;
-    for (int s0 = 0; s0 < rows; s0 += CR_SUB) {
-      const int sub = min(CR_SUB, rows - s0);
-      __syncthreads();
-      for (int i = threadIdx.x; i < sub * c2; i += OC_THREADS) Ls[i] = L[(size_t)s0 * c2 + i];
-      for (int i = threadIdx.x; i < sub * c1; i += OC_THREADS) Rs[i] = Rm[(size_t)s0 * c1 + i];
-      __syncthreads();
-      if (pairs <= 256) {
-        const int per = (sub + (OC_THREADS / 32) - 1) / (OC_THREADS / 32);
-        const int i0 = warp * per, i1 = min(sub, i0 + per);
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows * c2; i += OC_THREADS) Ls[i] = L[i];
+    for (int i = threadIdx.x; i < rows * c1; i += OC_THREADS) Rs[i] = Rm[i];
+    __syncthreads();
+    if (pairs <= 256) {
+      const int per = (rows + (OC_THREADS / 32) - 1) / (OC_THREADS / 32);
+      const int i0 = warp * per, i1 = min(rows, i0 + per);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int pr = lane + 32 * u;
-          if (pr < pairs) {
-            const int a = pr / c1, b = pr - a * c1;
-            float v = acc[u];
-            for (int i = i0; i < i1; ++i) v = fmaf(Ls[i * c2 + a], Rs[i * c1 + b], v);
-            acc[u] = v;
-          }
-        }
-      } else {                                     // ranks above 16: every thread its pairs over all rows
-        for (int pr = threadIdx.x; pr < pairs; pr += OC_THREADS) {
+      for (int u = 0; u < 8; ++u) {
+        const int pr = lane + 32 * u;
+        if (pr < pairs) {
           const int a = pr / c1, b = pr - a * c1;
           float v = 0.f;
-          for (int i = 0; i < sub; ++i) v = fmaf(Ls[i * c2 + a], Rs[i * c1 + b], v);
-          atomicAdd(c + pr, v);
+          for (int i = i0; i < i1; ++i) v = fmaf(Ls[i * c2 + a], Rs[i * c1 + b], v);
+          acc[u] = v;
         }
+      }
+    } else {                                       // ranks above 16: every thread its pairs over all rows
+      for (int pr = threadIdx.x; pr < pairs; pr += OC_THREADS) {
+        const int a = pr / c1, b = pr - a * c1;
+        float v = 0.f;
+        for (int i = 0; i < rows; ++i) v = fmaf(Ls[i * c2 + a], Rs[i * c1 + b], v);
+        atomicAdd(c + pr, v);
       }
     }
     if (pairs <= 256) {
@@ -1024,8 +1024,9 @@ k_corr_reduce(const ConefCorr* __restrict__ table, const int2* __restrict__ tile
   }
 }
 
-// k_corr_apply: T += sum_t coef_t X_t C_t.  A thread owns whole rows (its X row in registers, the small
-// C matrices in shared memory), so every row is one pass of wide loads and stores.
+// k_corr_apply: T += sum_t coef_t X_t C_t, one element of T per thread: loads and stores of T are whole lines,
+// and a row's X values are broadcast among the threads that share it.  (A thread with a whole row of T spread the
+// 4-byte accesses of a warp over 32 rows and kept 32 sums in registers.)
 __global__ void __launch_bounds__(OC_THREADS)
 k_corr_apply(const ConefCorr* __restrict__ table, const int2* __restrict__ tiles, float* __restrict__ Tb,
              const float* __restrict__ X0b, const float* __restrict__ X1b, const float* __restrict__ cbuf,
@@ -1034,33 +1035,27 @@ k_corr_apply(const ConefCorr* __restrict__ table, const int2* __restrict__ tiles
   const int2 t = tiles[blockIdx.x];
   const ConefCorr K = table[t.x];
   const int c1 = K.c1;
+  const int row0 = t.y * OC_ROWS + blockIdx.y * CR_SUB;
+  const int rows = min(CR_SUB, K.rows_t - row0);
+  if (rows <= 0) return;
   for (int term = 0; term < K.nterms; ++term) {
     const float* c = cbuf + ((size_t)t.x * 2 + term) * GRAM_STRIDE;
     for (int i = threadIdx.x; i < c1 * K.c2[term]; i += OC_THREADS) Csm[term][i] = c[i];
   }
   __syncthreads();
-  const int row0 = t.y * OC_ROWS;
-  const int rows = min(OC_ROWS, K.rows_t - row0);
   float* T = Tb + K.t_off + (size_t)row0 * c1;
-  for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
-    float out[OC_MAXR];
-#pragma unroll
-    for (int b = 0; b < OC_MAXR; ++b) out[b] = 0.f;
+  for (int e = threadIdx.x; e < rows * c1; e += OC_THREADS) {
+    const int i = e / c1, b = e - i * c1;
+    float out = 0.f;
     for (int term = 0; term < K.nterms; ++term) {
       const int c2 = K.c2[term];
       const float coef = term ? coef1 : coef0;
       const float* X = (term ? X1b : X0b) + K.x_off[term] + (size_t)(row0 + i) * c2;
-      for (int a = 0; a < c2; ++a) {
-        const float xa = coef * X[a];
-#pragma unroll
-        for (int b = 0; b < OC_MAXR; ++b)
-          if (b < c1) out[b] = fmaf(xa, Csm[term][a * c1 + b], out[b]);
-      }
+      const float* C = Csm[term] + b;
+#pragma unroll 8
+      for (int a = 0; a < c2; ++a) out = fmaf(coef * X[a], C[a * c1], out);
     }
-    float* trow = T + (size_t)i * c1;
-#pragma unroll
-    for (int b = 0; b < OC_MAXR; ++b)
-      if (b < c1) trow[b] += out[b];
+    T[e] += out;
   }
 }
 
@@ -1072,9 +1067,9 @@ extern "C" int conef_lowrank_correct(const ConefCorr* table, int nmats, const in
                                      cudaStream_t stream) {
   if (nmats <= 0 || n_reduce <= 0 || n_apply <= 0) return 0;
   CONEF_CUDA(cudaMemsetAsync(cbuf, 0, sizeof(float) * (size_t)nmats * 2 * GRAM_STRIDE, stream));
-  k_corr_reduce<<<n_reduce, OC_THREADS, 0, stream>>>(table, reduce_tiles, L0, R0, L1, R1, cbuf);
+  k_corr_reduce<<<dim3((unsigned)n_reduce, OC_ROWS / CR_SUB), OC_THREADS, 0, stream>>>(table, reduce_tiles, L0, R0, L1, R1, cbuf);
   CONEF_CHECK_LAUNCH("k_corr_reduce");
-  k_corr_apply<<<n_apply, OC_THREADS, 0, stream>>>(table, apply_tiles, T, X0, X1, cbuf, coef0, coef1);
+  k_corr_apply<<<dim3((unsigned)n_apply, OC_ROWS / CR_SUB), OC_THREADS, 0, stream>>>(table, apply_tiles, T, X0, X1, cbuf, coef0, coef1);
   CONEF_CHECK_LAUNCH("k_corr_apply");
   return 0;
 }

@@ -584,3 +584,48 @@ def test_lamb_slices_and_misaligned_tensors(shift):
                            1, clip)
         for got, w in zip((p.detach(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"]), want):
             assert float((got.double() - w).abs().max()) <= 1e-5 * float(w.abs().max()), (sizes[k], k)
+
+
+@pytest.mark.parametrize("c1,c2", [(1, 1), (4, 8), (8, 8), (3, 16), (20, 20), (32, 32)])
+def test_lowrank_correct_rows_and_ranks(c1, c2):
+    """T += sum_t coef_t X_t (L_t^T R_t) at row counts around the 128 rows of a CTA and the 512 of a chunk, one and
+    two terms, with ranks on both sides of the 256 products that a warp keeps.  Tolerance: 32-bit sums of up to 1,030
+    products times a sum of c2, measured against 64 bits relative to the result's largest entry."""
+    lib = native.lib()
+    shapes = [(1, 1), (127, 129), (128, 128), (129, 511), (513, 512), (1030, 513)]      # (rows of T, rows of L)
+    gen = torch.Generator().manual_seed(c1 * 64 + c2)
+    rand = lambda *s: torch.randn(*s, generator=gen)
+    tab = np.zeros(len(shapes), dtype=native.CORR_DTYPE)
+    T, X, L, R, want = [], [[], []], [[], []], [[], []], []
+    at = dict(t=0, x=[0, 0], l=[0, 0], r=[0, 0])
+    for k, (rt, rl) in enumerate(shapes):
+        tab[k]["t_off"], tab[k]["rows_t"], tab[k]["rows_l"], tab[k]["c1"], tab[k]["nterms"] = at["t"], rt, rl, c1, 1 + k % 2
+        t = rand(rt, c1)
+        w = t.double()
+        for term, coef in ((0, 0.5), (1, -1.0)):
+            x, l, rr = rand(rt, c2), rand(rl, c2), rand(rl, c1)
+            tab[k]["x_off"][term], tab[k]["l_off"][term], tab[k]["r_off"][term] = at["x"][term], at["l"][term], at["r"][term]
+            tab[k]["c2"][term] = c2
+            for name, lst, v in (("x", X, x), ("l", L, l), ("r", R, rr)):
+                lst[term].append(v.reshape(-1))
+                at[name][term] += v.numel()
+            if term <= k % 2:
+                w = w + coef * x.double() @ (l.double().t() @ rr.double())
+        T.append(t.reshape(-1))
+        at["t"] += t.numel()
+        want.append(w)
+    cat = lambda lst: torch.cat(lst).to(DEV)
+    Td, Xd, Ld, Rd = cat(T), [cat(x) for x in X], [cat(x) for x in L], [cat(x) for x in R]
+    tiles = lambda col: torch.tensor([(k, c) for k, s in enumerate(shapes) for c in range((s[col] + 511) // 512)],
+                                     dtype=torch.int32, device=DEV)
+    red, app = tiles(1), tiles(0)
+    cbuf = torch.zeros(len(shapes) * 2048, device=DEV)
+    tabd = native.upload_struct_array(tab, torch.device(DEV))
+    native.check(lib.conef_lowrank_correct(tabd.data_ptr(), len(shapes), red.data_ptr(), len(red), app.data_ptr(), len(app),
+                                           Td.data_ptr(), Xd[0].data_ptr(), Ld[0].data_ptr(), Rd[0].data_ptr(), 0.5,
+                                           Xd[1].data_ptr(), Ld[1].data_ptr(), Rd[1].data_ptr(), -1.0, cbuf.data_ptr(), _st()))
+    off = 0
+    for w in want:
+        got = Td[off : off + w.numel()].view_as(w).cpu().double()
+        off += w.numel()
+        assert float((got - w).abs().max()) <= 2e-5 * float(w.abs().max())
