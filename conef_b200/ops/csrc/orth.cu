@@ -296,26 +296,36 @@ constexpr long long ORTH_BARRIER_LIMIT = 2LL * 1000 * 1000;
 // Shifted Cholesky factor R of G (r x r, row stride RP + 1) by the first warp; see the file header.  R must
 // be zero on entry.  rd[c] = 1 / (R[c][c] + eps), or 0 for a column without a direction.  The rows are then
 // multiplied by (R + eps I)^-1 through a forward substitution per row (apply_factor), which needs no explicit
-// inverse: this serial section runs on one warp while the SM's other warps compete for issue slots, so its
-// cost is its instruction count (measured 3.5 us at r = 4 and 6 us at r = 8 with the inverse, per call).
+// inverse.  The section is a serial chain on one warp, so its cost is the latency of one step: lane c keeps
+// column c of G in registers and the warp eliminates row by row (the same subtractions in the same order as a
+// column-by-column factorisation), handing the new row of R round by shuffles: a step is a square root, a
+// division and one shuffle.  Reading G and R back from shared memory in loops over r took 6,500 cycles per call
+// at r = 8 and 3,000 at r = 4, more than half of the kernel, which went from 22 to 17 us per launch on a
+// BERT-large bucket of 29 MB (r = 8; with the Gram and store loops below).
 template <int RP>
 __device__ __forceinline__ void chol_factor(const float (*G)[RP + 1], float (*R)[RP + 1], float* rd, int r,
                                             float shift, float eps) {
   const int lane = threadIdx.x;
-  for (int j = 0; j < r; ++j) {
-    float d = G[j][j];
-    for (int k = 0; k < j; ++k) d -= R[k][j] * R[k][j];
-    const bool dead = !(G[j][j] > 0.f);
-    const float floor_d = shift * G[j][j];
-    if (!(d > floor_d)) d = floor_d;
-    const float rjj = dead ? 0.f : sqrtf(d);
-    if (lane == j) { R[j][j] = rjj; rd[j] = dead ? 0.f : 1.f / (rjj + eps); }
-    if (lane > j && lane < r) {
-      float v = G[j][lane];
-      for (int k = 0; k < j; ++k) v -= R[k][j] * R[k][lane];
-      R[j][lane] = dead ? 0.f : v / rjj;
+  float g[RP];                                   // g[k] = G[k][lane], of which k <= lane is used
+#pragma unroll
+  for (int k = 0; k < RP; ++k) g[k] = (lane < r && k <= lane) ? G[k][lane] : 0.f;
+  const float diag = lane < r ? G[lane][lane] : 0.f;
+#pragma unroll
+  for (int j = 0; j < RP; ++j) {
+    if (j < r) {
+      float d = __shfl_sync(0xffffffffu, g[j], j);
+      const float gjj = __shfl_sync(0xffffffffu, diag, j);
+      const bool dead = !(gjj > 0.f);
+      const float floor_d = shift * gjj;
+      if (!(d > floor_d)) d = floor_d;
+      const float rjj = dead ? 0.f : sqrtf(d);
+      const float row = dead ? 0.f : g[j] / rjj;      // R[j][lane] for lane > j
+      if (lane == j) { R[j][j] = rjj; rd[j] = dead ? 0.f : 1.f / (rjj + eps); }
+      if (lane > j && lane < r) R[j][lane] = row;
+#pragma unroll
+      for (int k = j + 1; k < RP; ++k)
+        if (k < r) g[k] = fmaf(-__shfl_sync(0xffffffffu, row, k), row, g[k]);
     }
-    __syncwarp();
   }
 }
 
@@ -636,14 +646,16 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
   // ---- load this CTA's rows (summing the peers' copies), four loads per thread (times the peers) in flight:
   //      one at a time, the 11 KB of a 720 x 4 block took 7 us ----
   const int nel = rows * r;
-  const bool vec4 = peer_bufs == nullptr && (r & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
+  const bool local = peer_bufs == nullptr || world <= 1;      // one rank: its slot buffer is an input like any other
+  const float* src = peer_bufs != nullptr && world <= 1 ? peer_bufs[0] + off : a;
+  const bool vec4 = local && (r & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
   if (vec4) {      // 16-byte loads of this GPU's own rows: an element group never straddles a row
     for (int q0 = 0; q0 < (nel >> 2); q0 += 4 * OC_THREADS) {
       float4 v4[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int q = q0 + u * OC_THREADS + threadIdx.x;
-        if (q < (nel >> 2)) v4[u] = __ldcg(reinterpret_cast<const float4*>(a) + q);
+        if (q < (nel >> 2)) v4[u] = __ldcg(reinterpret_cast<const float4*>(src) + q);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -663,10 +675,10 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
       const int i = base + u * OC_THREADS + threadIdx.x;
       v[u] = 0.f;
       if (i < nel) {
-        if (peer_bufs != nullptr) {
+        if (!local) {
           if (peers_ok) for (int p = 0; p < world; ++p) v[u] += ld_relaxed_sys_f32(peer_bufs[p] + off + i);
         } else {
-          v[u] = a[i];
+          v[u] = __ldcg(src + i);
         }
       }
     }
@@ -679,7 +691,6 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
       }
     }
   }
-  const int pairs = r * r;
   float* pk = packed ? packed + (which == 0 ? M.ppk_off : M.qpk_off) : nullptr;
   const bool project = X.tables != nullptr && which == 1 && pk != nullptr && M.tab_off >= 0;
   const int32_t* tab = project ? X.tables + M.tab_off : nullptr;
@@ -689,91 +700,100 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
 #pragma unroll 1
   for (int round = 0; round < 2; ++round) {
     __syncthreads();
-    // ---- Gram partial of this CTA's rows, fixed summation order: warps over row slices, then warps in order ----
-    if (pairs <= 256) {
+    // ---- Gram partial of this CTA's rows, fixed summation order: warps over row slices, then warps in order.
+    //      A warp covers the whole RP x RP matrix at once: each lane E neighbouring entries of one row of it, or,
+    //      where the matrix has fewer than 32 entries, the lanes take turns over the rows in NSUB groups.  One entry
+    //      per lane and as many passes over the rows as that takes: 1,300 cycles at 8 x 64 rows, 2,500 at 4 x 720 ----
+    if (PAIRS_MAX <= 256) {
+      constexpr int E = PAIRS_MAX > 32 ? PAIRS_MAX / 32 : 1;
+      constexpr int NSUB = PAIRS_MAX < 32 ? 32 / PAIRS_MAX : 1;
       const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
       const int per = (rows + (OC_THREADS / 32) - 1) / (OC_THREADS / 32);
       const int i0 = warp * per, i1 = min(rows, i0 + per);
-      for (int pr = lane; pr < pairs; pr += 32) {
-        const int ca = pr / r, cb = pr - ca * r;
-        float acc = 0.f;
-        for (int i = i0; i < i1; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
-        part[warp][pr] = acc;
+      const int sub = lane / (32 / NSUB), e0 = (lane % (32 / NSUB)) * E;
+      const float* xa = xs + e0 / RP;
+      const float* xb = xs + e0 % RP;
+      float acc[E];
+#pragma unroll
+      for (int q = 0; q < E; ++q) acc[q] = 0.f;
+#pragma unroll 4
+      for (int i = i0 + sub; i < i1; i += NSUB) {
+        const float va = xa[i * S];
+#pragma unroll
+        for (int q = 0; q < E; ++q) acc[q] = fmaf(va, xb[i * S + q], acc[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < E; ++q) {
+#pragma unroll
+        for (int o = 32 / NSUB; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+        if (sub == 0) part[warp][e0 + q] = acc[q];
       }
       __syncthreads();
-      if ((int)threadIdx.x < pairs) {
-        float acc = 0.f;
+      if ((int)threadIdx.x < PAIRS_MAX) {
+        float sum = 0.f;
 #pragma unroll
-        for (int w = 0; w < OC_THREADS / 32; ++w) acc += part[w][threadIdx.x];
-        gpart[round][threadIdx.x] = acc;
+        for (int w = 0; w < OC_THREADS / 32; ++w) sum += part[w][threadIdx.x];
+        gpart[round][threadIdx.x] = sum;
       }
     } else {
-      for (int pr = threadIdx.x; pr < pairs; pr += OC_THREADS) {
-        const int ca = pr / r, cb = pr - ca * r;
+      for (int pr = threadIdx.x; pr < PAIRS_MAX; pr += OC_THREADS) {
+        const int ca = pr / RP, cb = pr % RP;
         float acc = 0.f;
-        for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
+        if (ca < r && cb < r)
+          for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
         gpart[round][pr] = acc;
       }
     }
     cluster_sync_all();      // every CTA's partial of this round is in its shared memory
     // ---- the block's Gram matrix: the cluster's partials in rank order; factor; inverse ----
     for (int i = threadIdx.x; i < RP * (RP + 1); i += OC_THREADS) (&R[0][0])[i] = 0.f;
-    for (int pr = threadIdx.x; pr < pairs; pr += OC_THREADS) {
+    for (int pr = threadIdx.x; pr < PAIRS_MAX; pr += OC_THREADS) {
       float gv[OCL];
 #pragma unroll
       for (int c = 0; c < OCL; ++c) gv[c] = ld_dsmem_f32(&gpart[round][pr], (uint32_t)c);
       float acc = 0.f;
 #pragma unroll
       for (int c = 0; c < OCL; ++c) acc += gv[c];
-      G[pr / r][pr % r] = acc;
+      G[pr / RP][pr % RP] = acc;
     }
     __syncthreads();
     if (threadIdx.x < 32) chol_factor<RP>(G, R, rd, r, round == 0 ? ORTH_SHIFT : ORTH_SHIFT_FINAL, round == 0 ? eps : 0.f);
     __syncthreads();
     // ---- apply: every thread its rows ----
     for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
-      float av[RP];
+      float av[RP], yv[RP];
 #pragma unroll
       for (int k = 0; k < RP; ++k) av[k] = xs[i * S + k];
-      float psc = 0.f;
-      long long ph = 0;
-      if (round == 1 && project) {
-        const int e = tab[grow0 + i];
-        psc = unpack_sign(e) * X.alpha;
-        ph = unpack_bucket(e);
-      }
-      float yv[RP];
       apply_factor<RP>(av, R, rd, r, yv);
 #pragma unroll
-      for (int c = 0; c < RP; ++c) {
-        if (c < r) {
-          const float v = yv[c];
-          if (round == 0) {
-            xs[i * S + c] = v;
-          } else {
-            a[(size_t)i * r + c] = v;
-            if (packed) conef_pack_store(packed, M, which, grow0 + i, c, v, packed_np);
-            if (project) atomicAdd(zpk + conef_packed_offset(ph, c, packed_np), psc * v);
-          }
-        }
-      }
+      for (int c = 0; c < RP; ++c)
+        if (c < r) xs[i * S + c] = yv[c];
     }
   }
   // ---- columns that were exactly zero: fixed pseudo-random values instead (rare; not unrolled) ----
 #pragma unroll 1
   for (int c = 0; c < r; ++c) {
     if (R[c][c] > 0.f) continue;
-    for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
+    for (int i = threadIdx.x; i < rows; i += OC_THREADS) {      // the thread that wrote this row above
       float z[4];
       conef_philox_normal4(ORTH_REFILL_SEED + (unsigned long long)rec * 64ull + (unsigned long long)which * 32ull + c,
                            (uint64_t)(grow0 + i), z);
-      const float v = z[0] * refill_scale;
-      a[(size_t)i * r + c] = v;
-      if (packed) conef_pack_store(packed, M, which, grow0 + i, c, v, packed_np);
-      if (project) {
-        const int e = tab[grow0 + i];
-        atomicAdd(zpk + conef_packed_offset(unpack_bucket(e), c, packed_np), unpack_sign(e) * X.alpha * v);
-      }
+      xs[i * S + c] = z[0] * refill_scale;
+    }
+  }
+  __syncthreads();
+  // ---- results, one element per thread: neighbouring threads write neighbouring addresses, and a block of few
+  //      rows keeps the whole CTA busy (a thread with a row of its own issued its r packed stores and r atomics
+  //      one after another: 3,900 cycles at 8 x 64 rows) ----
+#pragma unroll 2
+  for (int e = threadIdx.x; e < nel; e += OC_THREADS) {
+    const int i = e / r, c = e - i * r;
+    const float v = xs[i * S + c];
+    a[e] = v;
+    if (packed) conef_pack_store(packed, M, which, grow0 + i, c, v, packed_np);
+    if (project) {
+      const int h = tab[grow0 + i];
+      atomicAdd(zpk + conef_packed_offset(unpack_bucket(h), c, packed_np), unpack_sign(h) * X.alpha * v);
     }
   }
   cluster_sync_all();      // no CTA leaves while a neighbour may still read its partials

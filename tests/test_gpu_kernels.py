@@ -629,3 +629,22 @@ def test_lowrank_correct_rows_and_ranks(c1, c2):
         got = Td[off : off + w.numel()].view_as(w).cpu().double()
         off += w.numel()
         assert float((got - w).abs().max()) <= 2e-5 * float(w.abs().max())
+
+
+@pytest.mark.parametrize("r", [1, 2, 3, 4, 5, 8, 11, 16, 17, 32])
+def test_orthogonalize_cluster_every_column_padding(r):
+    """The cluster form at every padding of the column count (1, 2, 4, 8, 16, 32 columns in registers) and at row
+    counts around the cluster's and the warps' shares, against 64 bits.  Tolerance: the Gram-Schmidt of a random
+    block is well conditioned; two rounds of 32-bit sums stay below 1e-4."""
+    gen = torch.Generator().manual_seed(r)
+    blocks = [torch.randn(n, r, generator=gen) for n in (max(r, 1), r + 7, 64 + r, 513, 2049, 8192)]
+    for i, (b, q) in enumerate(zip(blocks, _orth_on_device([b.clone() for b in blocks], cluster=True))):
+        if i == 0 and r > 1:      # square: the last column's direction is what is left over, badly conditioned
+            assert torch.isfinite(q).all()
+            continue
+        want = b.double()
+        ref.gram_schmidt_ref(want)
+        q = q.double()
+        torch.testing.assert_close(q.t() @ q, torch.eye(r, dtype=torch.float64), rtol=0, atol=1e-4)
+        if i > 1:
+            torch.testing.assert_close(q, want, rtol=0, atol=1e-4)
