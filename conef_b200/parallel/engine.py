@@ -105,6 +105,27 @@ def _status_words(device: torch.device) -> torch.Tensor:
     return t
 
 
+def decompress_rows(block_ctas, off_rows: int, off_width: int) -> int:
+    """Matrix rows per unit of the decompress kernels, in {8, 4, 2, 1}.
+
+    ``block_ctas(rows)``: CTAs of the block-layout kernel at that many rows.  A unit reads a group's Q rows once for
+    all its rows (at rank 4, 512 bytes beside 128 per row), so more rows are less traffic and fewer instructions per
+    element for as long as the launch fills the device.  Measured in us, 1 / 2 / 4 / 8 rows (CTAs at 8 rows):
+    two 640 x 5760 at rank 4 45 / 31 / 20 / 17 (360), one of them 24 / 17 / 13 / 13 (180), 4096 x 1024 at rank 8
+    35 / 23 / 16 / 17 (192), 1024 x 1024 9.8 / 9.0 / 8.9 / 11 (48), 512 x 1024 8.0 / 7.6 / 8.7 / 11 (24),
+    four 64 x 1152 7.7 / 8.1 / 9.3 / 12 (12): eight from two CTAs per SM on, four or two from 96 CTAs on.
+    ``off_rows`` / ``off_width``: rows and widest sketch of the matrices that go to the column-order kernels (dense
+    or no error feedback among them: width 0), whose tile is a block of rows with one accumulator row each in shared
+    memory: the most that fit while every SM still gets a few CTAs."""
+    for rows, ctas in ((8, 2 * 148), (4, 96), (2, 96)):
+        if off_rows == 0 and block_ctas(rows) >= ctas:
+            return rows
+        if off_rows and rows * off_width * 4 <= SMEM_BUDGET // 4 and \
+                (off_rows // rows >= 3 * 148 or block_ctas(rows) >= ctas):
+            return rows
+    return 1
+
+
 class _EngineBase:
     def __init__(self, device):
         self.device = device
@@ -335,32 +356,29 @@ class PowerSGDEngine(_EngineBase):
         max_tiles = max((n for _, n, _ in self.orth_tiles.values()), default=1)
         self.gram = torch.zeros(max(max_tiles, 1) * 2 * 1024, device=dev, dtype=torch.float32)
 
-        # decompress: rows per CTA in {8, 4, 2, 1}: the most that fit in shared memory (one
-        # accumulator row of the sketch width per matrix row) while still giving every SM a few CTAs
+        # decompress: matrices on the block layout of the hash come first: they run on the atomics-free kernel,
+        # whose tile is a chunk of eight (row block, cell block) units, one per warp; the others by row block
         maxW = max(self.widths, default=0)
         if maxW * 4 > SMEM_BUDGET:
             raise native.NativeError(f"sketch width {maxW} does not fit in shared memory")
-        total_rows = sum(e.n for e in plan.mats)
-        self.d_rows = 1
-        for cand in (8, 4, 2):
-            if cand * maxW * 4 <= SMEM_BUDGET // 4 and total_rows // cand >= 3 * 148:
-                self.d_rows = cand
-                break
-        if os.environ.get("CONEF_D_ROWS"):
-            self.d_rows = int(os.environ["CONEF_D_ROWS"])
-        self.d_smem = self.d_rows * maxW * 4
-        # matrices on the block layout of the hash first: they run on the atomics-free kernel, whose tile
-        # is a chunk of eight (row block, cell block) units, one per warp; the others by row block
         on_blocks = [int(mats[k]["cb_off"]) >= 0 for k in range(nm)]
         self.d_rbu = int(os.environ.get("CONEF_D_RBU", "1"))
 
-        def units(e, W):      # (row blocks of a unit, cell block); matrices with more than 32 windows: one row block
+        def units(e, W, rows):      # (row blocks of a unit, cell block); more than 32 windows: one row block
             nb = W // 32
             windows = math.ceil(math.ceil(e.m / 32) / nb)
             per_unit = self.d_rbu if windows <= 32 else 1
-            return math.ceil(math.ceil(e.n / self.d_rows) / per_unit) * nb
+            return math.ceil(math.ceil(e.n / rows) / per_unit) * nb
+        on_list = [(e, self.widths[k]) for k, e in enumerate(plan.mats) if on_blocks[k]]
+        off_rows = sum(e.n for k, e in enumerate(plan.mats) if not on_blocks[k])
+        off_W = max((w for k, w in enumerate(self.widths) if not on_blocks[k]), default=0)
+        self.d_rows = decompress_rows(lambda rows: sum(math.ceil(units(e, W, rows) / 8) for e, W in on_list),
+                                      off_rows, off_W)
+        if os.environ.get("CONEF_D_ROWS"):
+            self.d_rows = int(os.environ["CONEF_D_ROWS"])
+        self.d_smem = self.d_rows * off_W * 4
         d_tiles = [(k, ch) for k, e in enumerate(plan.mats) if on_blocks[k]
-                   for ch in range(math.ceil(units(e, self.widths[k]) / 8))]
+                   for ch in range(math.ceil(units(e, self.widths[k], self.d_rows) / 8))]
         self.d_nblk = len(d_tiles)
         d_tiles += [(k, rb) for k, e in enumerate(plan.mats) if not on_blocks[k]
                     for rb in range(math.ceil(e.n / self.d_rows))]
