@@ -105,6 +105,34 @@ def _status_words(device: torch.device) -> torch.Tensor:
     return t
 
 
+def split_k(mn: int, K: int, extent: int):
+    """(output tiles, K extent of a CTA, CTAs per output tile) of one (mn x K) product at a target extent."""
+    splits = max(1, round(K / extent))
+    klen = math.ceil(math.ceil(K / splits) / 32) * 32
+    return math.ceil(mn / 128), klen, math.ceil(K / klen)
+
+
+def one_wave_extent(dims, slots: int = TARGET_CTAS, shortest: int = 128):
+    """The shortest K extent (a multiple of 32) at which the tensor-core tiles of all (mn, K) products of a launch
+    are resident at once, or None when no extent does that.  All CTAs of a launch do about the same work, so a few
+    more than the device holds (two per SM) cost a second round as long as the first.  Measured in us, P = M Q and
+    Q = M^T P, against three waves of CTAs with extents of 384 to 1,024: one 512 x 512 matrix 8.1, 7.8 -> 4.7, 4.8
+    (20 CTAs of 128 instead of 10 of 256 to 512), 30528 x 1024 41, 42 -> 31, 26 (extent 928 instead of 384), two
+    640 x 5760 8.2, 7.8 -> 7.7, 7.8 (300 CTAs of 224 for the second product would take 10.2)."""
+    if not dims:
+        return None
+    longest = max(K for _, K in dims)
+    work = sum(math.ceil(mn / 128) * K for mn, K in dims)
+    extent = max(shortest, int(0.6 * work / slots) // 32 * 32)      # below this there are too many for certain
+    for _ in range(64):
+        if sum(t * s for t, _, s in (split_k(mn, K, extent) for mn, K in dims)) <= slots:
+            return extent
+        if extent > 2 * longest:
+            return None
+        extent += max(32, extent // 512 * 32)
+    return None
+
+
 def decompress_rows(block_ctas, off_rows: int, off_width: int) -> int:
     """Matrix rows per unit of the decompress kernels, in {8, 4, 2, 1}.
 
@@ -468,30 +496,32 @@ class PowerSGDEngine(_EngineBase):
         good = [k for k in range(nrec) if self.tc_ok[k]]
         bad = [k for k in range(nrec) if not self.tc_ok[k]]
 
+        # used when no extent fits the launch into one wave of CTAs, or when one of the variables is set
+        tuned = any(v in os.environ for v in ("CONEF_TC_WAVES", "CONEF_TC_MIN_K", "CONEF_TC_MAX_K"))
         waves = float(os.environ.get("CONEF_TC_WAVES", 3))
         min_k = int(os.environ.get("CONEF_TC_MIN_K", 384))
         max_k = int(os.environ.get("CONEF_TC_MAX_K", 1024))
 
         def split_tiles(mode):
             # mode 0 (P): output rows = n, K = m.  mode 1 (Q): output rows = m, K = n.
-            # Every tile gets about the same K extent, chosen so that the launch has a few
-            # waves of CTAs (two CTAs fit on an SM) without making tiles too short.
+            # Every tile gets about the same K extent: the shortest with which all CTAs are resident at once (two
+            # fit on an SM), or, with more output tiles than that, an equal share of the work for that many.
             def view(k):        # (output rows, K) of record k, in its folded view when it has one
                 n_, m_, f = int(recs[k]["n"]), int(recs[k]["m"]), max(1, int(recs[k]["fold"]))
                 return (m_ * f, n_ // f) if mode else (n_ // f, m_ * f)
             dims = [view(k) for k in good]
-            work = sum(math.ceil(mn / 128) * K for mn, K in dims)
-            klen_t = work / max(1.0, waves * TARGET_CTAS)
-            klen_t = int(min(max_k, max(min_k, math.ceil(klen_t / 32) * 32)))
+            klen_t = None if tuned else one_wave_extent(dims)
+            if klen_t is None:
+                work = sum(math.ceil(mn / 128) * K for mn, K in dims)
+                klen_t = work / max(1.0, (waves if tuned else 1.0) * TARGET_CTAS)
+                klen_t = int(min(max_k if tuned else 1 << 30, max(min_k, math.ceil(klen_t / 32) * 32)))
             tiles = []
             for k, (mn, K) in zip(good, dims):
-                splits = max(1, round(K / klen_t))
-                klen = math.ceil(math.ceil(K / splits) / 32) * 32
-                splits = math.ceil(K / klen)
+                mblocks, klen, splits = split_k(mn, K, klen_t)
                 shared = self.fused_err if mode == 0 else self.ef_mode == native.EF_DENSE
                 folded_q = mode == 1 and int(recs[k]["fold"]) > 1       # its row blocks add into one Q block
                 flag = (1 << 30) if (splits > 1 or shared or folded_q) else 0
-                for mb in range(math.ceil(mn / 128)):
+                for mb in range(mblocks):
                     for sp in range(splits):
                         tiles.append((k | flag, mb * 128, sp * klen, klen))
             t = torch.from_numpy(np.asarray(tiles, dtype=np.int32).reshape(-1, 4)).to(dev) if tiles else None
