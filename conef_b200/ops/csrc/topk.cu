@@ -61,16 +61,28 @@ k_topk_hist(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, c
     if (h[i]) atomicAdd(g + i, h[i]);
 }
 
-// One CTA (one warp) per matrix: find the bin, counted from the top, in which the cumulative count
-// reaches `remaining`; append it to the prefix, keep what is still wanted inside that bin, and clear
-// the histogram for the next pass.
-__global__ void k_topk_scan(const ConefMat* __restrict__ mats, TopkState* __restrict__ st, uint32_t* __restrict__ hist,
-                            int pass, float ratio) {
-  const int k = blockIdx.x, lane = threadIdx.x;
-  const int bins = pass == 0 ? TK_BINS : 1024, shift = pass == 0 ? 11 : 10;
-  uint32_t* g = hist + (size_t)k * TK_BINS;
+// One CTA per matrix: find the bin, counted from the top, in which the cumulative count reaches
+// `remaining`; append it to the prefix, keep what is still wanted inside that bin, and clear the
+// histogram for the next pass.  Pure latency: a thread owns BINS / SCAN_THREADS neighbouring bins, which
+// it holds in registers from the one round of loads on (one warp with 32 to 64 bins per lane, read twice,
+// took 5.2 us per launch on a Transformer bucket, now 1.5 to 2.2).
+constexpr int SCAN_THREADS = 256;
+template <int PASS>
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_topk_scan(const ConefMat* __restrict__ mats, TopkState* __restrict__ st, uint32_t* __restrict__ hist, float ratio) {
+  constexpr int BINS = PASS == 0 ? TK_BINS : 1024, SHIFT = PASS == 0 ? 11 : 10;
+  constexpr int PER = BINS / SCAN_THREADS;
+  __shared__ uint32_t warp_total[SCAN_THREADS / 32];
+  const int k = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // thread 0 owns the top bins
+  uint32_t* g = hist + (size_t)k * TK_BINS + (BINS - PER * (tid + 1));
+  uint32_t c[PER];                          // ascending bins
+#pragma unroll
+  for (int i = 0; i < PER; ++i) c[i] = g[i];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) g[i] = 0u;
   TopkState s = st[k];
-  if (pass == 0) {
+  if (PASS == 0) {
     const long long numel = (long long)mats[k].n * mats[k].m;
     long long want = (long long)(0.5 * (double)ratio * (double)numel);
     if (want < 1) want = 1;
@@ -78,39 +90,41 @@ __global__ void k_topk_scan(const ConefMat* __restrict__ mats, TopkState* __rest
     s.prefix = 0;
     s.remaining = (uint32_t)want;
   }
-  const int per = bins / 32;               // lane 0 owns the top bins
-  const int top = bins - 1 - lane * per;   // highest bin of this lane
   uint32_t mine = 0;
-  for (int i = 0; i < per; ++i) mine += g[top - i];
-  uint32_t incl = mine;                     // inclusive scan over lanes (top lanes first)
+#pragma unroll
+  for (int i = 0; i < PER; ++i) mine += c[i];
+  uint32_t incl = mine;                     // inclusive scan over threads (top bins first)
+#pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
-  const uint32_t before = incl - mine;
-  const bool here = before < s.remaining && incl >= s.remaining;
-  const unsigned who = __ballot_sync(0xffffffffu, here);
-  uint32_t digit = 0, rem = s.remaining;
-  if (who == 0) {                           // fewer candidates than wanted (cannot happen for pass 0): keep all
-    digit = 0;
-    rem = 0;
-  } else {
-    const int src = __ffs(who) - 1;
-    if (lane == src) {
-      uint32_t acc = before;
-      for (int i = 0; i < per; ++i) {
-        const uint32_t c = g[top - i];
-        if (acc + c >= s.remaining) { digit = (uint32_t)(top - i); rem = s.remaining - acc; break; }
-        acc += c;
+  if (lane == 31) warp_total[warp] = incl;
+  __syncthreads();                          // also: every thread has read the state
+  uint32_t total = 0;
+#pragma unroll
+  for (int w = 0; w < SCAN_THREADS / 32; ++w) {
+    if (w < warp) incl += warp_total[w];
+    total += warp_total[w];
+  }
+  uint32_t before = incl - mine;
+  // Exactly one thread holds the bin; fewer candidates than wanted (cannot happen in the first pass): keep all
+  const bool none = !(total >= s.remaining && s.remaining > 0);
+  if (none ? tid == 0 : (before < s.remaining && incl >= s.remaining)) {
+    uint32_t digit = 0, rem = 0;
+    if (!none) {
+      bool found = false;
+#pragma unroll
+      for (int i = PER - 1; i >= 0; --i) {  // from the top
+        if (!found && before + c[i] >= s.remaining) {
+          digit = (uint32_t)(BINS - PER * (tid + 1) + i);
+          rem = s.remaining - before;
+          found = true;
+        }
+        before += c[i];
       }
     }
-    digit = __shfl_sync(0xffffffffu, digit, src);
-    rem = __shfl_sync(0xffffffffu, rem, src);
-  }
-  __syncwarp();
-  for (int i = lane; i < bins; i += 32) g[i] = 0;
-  if (lane == 0) {
-    s.prefix = (s.prefix << shift) | digit;
+    s.prefix = (s.prefix << SHIFT) | digit;
     s.remaining = rem;
     st[k] = s;
   }
@@ -161,15 +175,15 @@ extern "C" int conef_topk_keep(const ConefMat* mats, int nmats, const int2* tile
   TopkState* st = reinterpret_cast<TopkState*>(scratch + (size_t)nmats * TK_BINS);
   k_topk_hist<0><<<ntiles, TK_THREADS, 0, stream>>>(mats, tiles, err, st, hist);
   CONEF_CHECK_LAUNCH("k_topk_hist<0>");
-  k_topk_scan<<<nmats, 32, 0, stream>>>(mats, st, hist, 0, ratio);
+  k_topk_scan<0><<<nmats, SCAN_THREADS, 0, stream>>>(mats, st, hist, ratio);
   CONEF_CHECK_LAUNCH("k_topk_scan");
   k_topk_hist<1><<<ntiles, TK_THREADS, 0, stream>>>(mats, tiles, err, st, hist);
   CONEF_CHECK_LAUNCH("k_topk_hist<1>");
-  k_topk_scan<<<nmats, 32, 0, stream>>>(mats, st, hist, 1, ratio);
+  k_topk_scan<1><<<nmats, SCAN_THREADS, 0, stream>>>(mats, st, hist, ratio);
   CONEF_CHECK_LAUNCH("k_topk_scan");
   k_topk_hist<2><<<ntiles, TK_THREADS, 0, stream>>>(mats, tiles, err, st, hist);
   CONEF_CHECK_LAUNCH("k_topk_hist<2>");
-  k_topk_scan<<<nmats, 32, 0, stream>>>(mats, st, hist, 2, ratio);
+  k_topk_scan<2><<<nmats, SCAN_THREADS, 0, stream>>>(mats, st, hist, ratio);
   CONEF_CHECK_LAUNCH("k_topk_scan");
   k_topk_apply<<<ntiles, TK_THREADS, 0, stream>>>(mats, tiles, err, st);
   CONEF_CHECK_LAUNCH("k_topk_apply");

@@ -648,3 +648,33 @@ def test_orthogonalize_cluster_every_column_padding(r):
         torch.testing.assert_close(q.t() @ q, torch.eye(r, dtype=torch.float64), rtol=0, atol=1e-4)
         if i > 1:
             torch.testing.assert_close(q, want, rtol=0, atol=1e-4)
+
+
+@pytest.mark.parametrize("ratio", [1e-9, 0.4, 1.0, 2.0])
+def test_grouped_topk_threshold_at_both_ends(ratio):
+    """The bin search at its ends: one entry kept, all kept, all entries equal, and magnitudes spread over the whole
+    exponent range (the threshold's digits then lie anywhere in the histograms)."""
+    lib = native.lib()
+    gen = torch.Generator().manual_seed(17)
+    n = 40_000
+    flat = [torch.full((n,), -0.75), torch.randn(n, generator=gen) * 10.0 ** (60 * torch.rand(n, generator=gen) - 30),
+            torch.arange(1, n + 1).float(), torch.tensor([3.0])]
+    mats = np.zeros(len(flat), dtype=native.MAT_DTYPE)
+    ch, off, tiles = lib.conef_topk_chunk(), 0, []
+    for k, f in enumerate(flat):
+        mats[k]["g_off"], mats[k]["n"], mats[k]["m"] = off, 1, f.numel()
+        tiles += [(k, c) for c in range((f.numel() + ch - 1) // ch)]
+        off += f.numel()
+    err = torch.cat(flat).to(DEV)
+    tl = torch.tensor(tiles, dtype=torch.int32, device=DEV)
+    scratch = torch.zeros(len(flat) * 2050, dtype=torch.int32, device=DEV)
+    md = native.upload_struct_array(mats, DEV)
+    native.check(lib.conef_topk_keep(md.data_ptr(), len(flat), tl.data_ptr(), len(tiles), err.data_ptr(), ratio,
+                                     scratch.data_ptr(), _st()))
+    off = 0
+    for f in flat:
+        keep = min(f.numel(), max(1, int(0.5 * ratio * f.numel())))
+        limit = f.abs().sort(descending=True).values[keep - 1]
+        torch.testing.assert_close(err[off : off + f.numel()].cpu(), torch.where(f.abs() >= limit, f, 0.0), rtol=0, atol=0)
+        off += f.numel()
+    assert int(scratch[: len(flat) * 2048].abs().sum()) == 0      # histograms left clean for the next call
