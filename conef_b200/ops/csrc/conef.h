@@ -144,6 +144,13 @@ int conef_sketch3_query(float* mat, const float* cs0, const float* cs1, const fl
 int conef_sketch3_update(const float* vec, float* cs0, float* cs1, float* cs2,
                          const int32_t* t0, const int32_t* t1, const int32_t* t2,
                          int N, int D, int W, float beta, cudaStream_t stream);
+// Every matrix of a bucket in one launch (per 32 matrices).  desc (host): ten numbers per matrix {cs0, cs1, cs2,
+// t0, t1, t2 (device addresses), offset in the bucket, N, D, W}.  query: work += estimates, the sums copied into
+// `before` as well; update: the sketches take in before - after.
+int conef_sketch3_query_group(float* work, float* before, const long long* desc, int nmats, float alpha,
+                              cudaStream_t stream);
+int conef_sketch3_update_group(const float* before, const float* after, const long long* desc, int nmats, float beta,
+                               cudaStream_t stream);
 
 // ---- grouped PowerSGD pipeline, SIMT (powersgd.cu) --------------------------
 // P_i (+)= A_i Q_i for every record: A_i is a matrix of the bucket (src 0) or of the

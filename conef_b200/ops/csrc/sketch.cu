@@ -219,6 +219,139 @@ extern "C" int conef_sketch3_update(const float* vec, float* cs0, float* cs1, fl
   return 0;
 }
 
+// All the matrices of a bucket in one launch.  The matrices arrive by value in the kernel's parameters (72 bytes
+// each), so that nothing is uploaded or kept between calls and a launch can be captured; a bucket with more than
+// SK3_GROUP of them takes another launch.  A small network's bucket is launch-bound: two launches and their host
+// calls per matrix, a clone of the bucket and its difference took
+// 533 us per hook call on ResNet-20's twelve matrices; the grouped form takes 148 us (kernels 112 -> 9 us).
+constexpr int SK3_GROUP = 32;
+struct Sk3Mat {
+  float* cs[3];
+  const int32_t* t[3];
+  long long off;      // first element in the bucket
+  int N, D, W;
+  int row_end;        // rows of this matrix and those before it
+};
+struct Sk3Group {
+  int n;
+  Sk3Mat m[SK3_GROUP];
+};
+__device__ __forceinline__ int sk3_find(const Sk3Group& g, int row, int& local) {
+  int k = 0, first = 0;
+  while (row >= g.m[k].row_end) first = g.m[k++].row_end;      // row < m[n - 1].row_end
+  local = row - first;
+  return k;
+}
+
+// One CTA per matrix row.  work += alpha-weighted estimate; `before` gets a copy of the result.
+__global__ void __launch_bounds__(256)
+k_sketch3_query_group(const __grid_constant__ Sk3Group g, float* __restrict__ work, float* __restrict__ before,
+                      float alpha) {
+  int row;
+  const Sk3Mat& M = g.m[sk3_find(g, blockIdx.x, row)];
+  const size_t base = (size_t)row * M.W, at = (size_t)M.off + (size_t)row * M.D;
+  const float *c0 = M.cs[0] + base, *c1 = M.cs[1] + base, *c2 = M.cs[2] + base;
+#pragma unroll 2
+  for (int j = threadIdx.x; j < M.D; j += 256) {
+    const int e0 = M.t[0][j], e1 = M.t[1][j], e2 = M.t[2][j];
+    const float a = alpha * unpack_sign(e0) * c0[unpack_bucket(e0)];
+    const float b = alpha * unpack_sign(e1) * c1[unpack_bucket(e1)];
+    const float c = alpha * unpack_sign(e2) * c2[unpack_bucket(e2)];
+    const float v = work[at + j] + median3(a, b, c);
+    work[at + j] = v;
+    before[at + j] = v;
+  }
+}
+
+// One CTA per matrix row; the vector that enters the sketch is before - after.
+__global__ void __launch_bounds__(256)
+k_sketch3_update_group(const __grid_constant__ Sk3Group g, const float* __restrict__ before,
+                       const float* __restrict__ after, float beta) {
+  extern __shared__ float sm[];
+  int row;
+  const Sk3Mat& M = g.m[sk3_find(g, blockIdx.x, row)];
+  const int W = M.W;
+  float* old = sm;
+  float* acc = sm + 3 * (size_t)W;
+  const size_t base = (size_t)row * W, at = (size_t)M.off + (size_t)row * M.D;
+  for (int i = threadIdx.x; i < W; i += 256) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      old[q * W + i] = M.cs[q][base + i];
+      acc[q * W + i] = 0.f;
+    }
+  }
+  __syncthreads();
+  const float k = -(1.f - beta);
+#pragma unroll 2
+  for (int j = threadIdx.x; j < M.D; j += 256) {
+    const int e0 = M.t[0][j], e1 = M.t[1][j], e2 = M.t[2][j];
+    const int h0 = unpack_bucket(e0), h1 = unpack_bucket(e1), h2 = unpack_bucket(e2);
+    const float s0 = unpack_sign(e0), s1 = unpack_sign(e1), s2 = unpack_sign(e2);
+    const float u = median3(k * s0 * old[h0], k * s1 * old[W + h1], k * s2 * old[2 * W + h2]) +
+                    (before[at + j] - after[at + j]);
+    atomicAdd(&acc[h0], s0 * u);
+    atomicAdd(&acc[W + h1], s1 * u);
+    atomicAdd(&acc[2 * W + h2], s2 * u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < W; i += 256)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) M.cs[q][base + i] = old[q * W + i] + acc[q * W + i];
+}
+
+// desc: ten numbers per matrix {cs0, cs1, cs2, t0, t1, t2 (device addresses), offset, N, D, W}.  Fills `g` with up
+// to SK3_GROUP non-empty matrices from `*next` on; returns the rows of the group (0: done, -1: too many).
+static long long sk3_group(const long long* desc, int nmats, int* next, Sk3Group* g, int* max_w) {
+  long long rows = 0;
+  g->n = 0;
+  *max_w = 0;
+  for (; *next < nmats && g->n < SK3_GROUP; ++*next) {
+    const long long* d = desc + (size_t)*next * 10;
+    if (d[7] <= 0 || d[8] <= 0) continue;
+    Sk3Mat& M = g->m[g->n++];
+    for (int q = 0; q < 3; ++q) {
+      M.cs[q] = reinterpret_cast<float*>((uintptr_t)d[q]);
+      M.t[q] = reinterpret_cast<const int32_t*>((uintptr_t)d[3 + q]);
+    }
+    M.off = d[6];
+    M.N = (int)d[7]; M.D = (int)d[8]; M.W = (int)d[9];
+    rows += d[7];
+    if (rows > 0x7fffffffLL) return -1;
+    M.row_end = (int)rows;
+    if (M.W > *max_w) *max_w = M.W;
+  }
+  return rows;
+}
+
+extern "C" int conef_sketch3_query_group(float* work, float* before, const long long* desc, int nmats, float alpha,
+                                         cudaStream_t stream) {
+  Sk3Group g;
+  int next = 0, max_w = 0;
+  for (long long rows; (rows = sk3_group(desc, nmats, &next, &g, &max_w)) != 0;) {
+    if (rows < 0) { conef_set_error("sketch3_query_group: too many rows"); return 2; }
+    k_sketch3_query_group<<<(unsigned)rows, 256, 0, stream>>>(g, work, before, alpha);
+    CONEF_CHECK_LAUNCH("k_sketch3_query_group");
+  }
+  return 0;
+}
+
+extern "C" int conef_sketch3_update_group(const float* before, const float* after, const long long* desc, int nmats,
+                                          float beta, cudaStream_t stream) {
+  Sk3Group g;
+  int next = 0, max_w = 0;
+  for (long long rows; (rows = sk3_group(desc, nmats, &next, &g, &max_w)) != 0;) {
+    if (rows < 0) { conef_set_error("sketch3_update_group: too many rows"); return 2; }
+    const size_t smem = (size_t)max_w * 6 * sizeof(float);
+    if (smem > 200 * 1024) { conef_set_error("sketch3_update_group: W=%d does not fit in shared memory", max_w); return 2; }
+    if (smem > 48 * 1024)
+      CONEF_CUDA(cudaFuncSetAttribute(k_sketch3_update_group, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    k_sketch3_update_group<<<(unsigned)rows, 256, smem, stream>>>(g, before, after, beta);
+    CONEF_CHECK_LAUNCH("k_sketch3_update_group");
+  }
+  return 0;
+}
+
 // ---------------------------------------------------------------------------
 // The sparse sign matrix H (m x W, one entry per row: H[j, h_j] = s_j) applied to the
 // small PowerSGD factors, grouped over the matrices of a bucket.  With the sketch S,

@@ -147,6 +147,8 @@ _SIGNATURES = {
     "conef_sketch_update": ([vp, vp, C.c_int, vp, vp, C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
     "conef_sketch3_query": ([vp] * 7 + [C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
     "conef_sketch3_update": ([vp] * 7 + [C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
+    "conef_sketch3_query_group": ([vp] * 3 + [C.c_int, C.c_float, vp], C.c_int),
+    "conef_sketch3_update_group": ([vp] * 3 + [C.c_int, C.c_float, vp], C.c_int),
     "conef_psgd_p": ([vp, vp, C.c_int, vp, vp, vp, vp, C.c_int, C.c_int, vp], C.c_int),
     "conef_sketch_project": ([vp, C.c_int, C.c_int, vp, vp, C.c_float, C.c_int, vp], C.c_int),
     "conef_psgd_q": ([vp, vp, C.c_int, vp, vp, vp, vp, C.c_int, vp], C.c_int),

@@ -21,6 +21,7 @@ blocks the host once per bucket, communication/powerSGD_hook.py:552-553).
 """
 from __future__ import annotations
 
+import ctypes
 import logging
 import math
 import os
@@ -30,7 +31,7 @@ import numpy as np
 import torch
 import torch.distributed as dist
 
-from ..compressors import DenseCS, Quant8Error, tables_for
+from ..compressors import DenseCS, DenseCSHash3, Quant8Error, tables_for
 from ..compressors.count_sketch import block_csr_for
 from ..compressors.count_sketch import HalfDenseCS
 from ..ops import native
@@ -152,6 +153,30 @@ def decompress_rows(block_ctas, off_rows: int, off_width: int) -> int:
                 (off_rows // rows >= 3 * 148 or block_ctas(rows) >= ctas):
             return rows
     return 1
+
+
+def sketch3_group(comps, mats, work: torch.Tensor):
+    """Descriptors of the grouped three-row sketch kernels (csrc/sketch.cu), or None when a store of the bucket is
+    something else (or lives elsewhere).  Built anew on every call: a user may replace a store or its tensors."""
+    if not mats or work.dtype != torch.float32 or not work.is_contiguous() or not native.use_native(work):
+        return None
+    flat, tables = [], {}
+    for cnt, e in enumerate(mats):
+        c = comps[cnt]
+        if type(c) is not DenseCSHash3 or c.N != e.n or c.D != e.m:
+            return None
+        for cs in (c.cs0, c.cs1, c.cs2):
+            if cs.dtype != torch.float32 or cs.device != work.device or not cs.is_contiguous() \
+                    or cs.numel() != c.N * c.range:
+                return None
+            flat.append(cs.data_ptr())
+        key = (c.D, c.range, *(v for seed in c.seeds for v in seed))
+        tabs = tables.get(key)
+        if tabs is None:
+            tabs = tables[key] = [t[2].data_ptr() for t in c._tables()]      # the tables are cached per device
+        flat += tabs
+        flat += (e.g_off, c.N, c.D, c.range)
+    return (ctypes.c_longlong * len(flat))(*flat)
 
 
 class _EngineBase:
@@ -863,9 +888,15 @@ class PowerSGDEngine(_EngineBase):
         copy = None
         if self.external:
             comps = state.error_dict[bidx]
-            for cnt, e in enumerate(plan.mats):
-                comps[cnt].query(work[e.g_off : e.g_off + e.numel], alpha)
-            copy = work.clone()
+            group = sketch3_group(comps, plan.mats, work)
+            if group is not None:
+                copy = torch.empty_like(work)
+                native.check(lib.conef_sketch3_query_group(wp, copy.data_ptr(), group, nm, float(alpha), st),
+                             "sketch3_query_group")
+            else:
+                for cnt, e in enumerate(plan.mats):
+                    comps[cnt].query(work[e.g_off : e.g_off + e.numel], alpha)
+                copy = work.clone()
 
         pmem, qmem, fresh = self._pq_memory(state, bidx)
         eps = float(getattr(state, "orthogonalization_epsilon", 0) or 0)
@@ -873,10 +904,14 @@ class PowerSGDEngine(_EngineBase):
         self._run_native(state, work, alpha, beta, fresh, eps, st)
 
         if self.external:
-            copy.sub_(work)
-            comps = state.error_dict[bidx]
-            for cnt, e in enumerate(plan.mats):
-                comps[cnt].update(copy[e.g_off : e.g_off + e.numel], beta)
+            if group is not None:
+                native.check(lib.conef_sketch3_update_group(copy.data_ptr(), wp, group, nm, float(beta), st),
+                             "sketch3_update_group")
+            else:
+                copy.sub_(work)
+                comps = state.error_dict[bidx]
+                for cnt, e in enumerate(plan.mats):
+                    comps[cnt].update(copy[e.g_off : e.g_off + e.numel], beta)
         if self.variant == "batched":
             buf.copy_(work[: self.buf_numel])
         if not getattr(state, "warm_start", False) or self.variant == "unbiased":

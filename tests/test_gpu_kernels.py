@@ -678,3 +678,49 @@ def test_grouped_topk_threshold_at_both_ends(ratio):
         torch.testing.assert_close(err[off : off + f.numel()].cpu(), torch.where(f.abs() >= limit, f, 0.0), rtol=0, atol=0)
         off += f.numel()
     assert int(scratch[: len(flat) * 2048].abs().sum()) == 0      # histograms left clean for the next call
+
+
+@pytest.mark.parametrize("shapes,size", [([(1, 1)], 0.1), ([(7, 33), (64, 576), (5, 255), (3, 256), (2, 257)], 0.1),
+                                         ([(3, 40 + k) for k in range(33)], 0.5), ([(2, 9000)], 0.9)],
+                         ids=["one", "edges", "two_groups", "opt_in_smem"])
+def test_grouped_sketch3_matches_reference(shapes, size):
+    """The grouped three-row sketch kernels against the PyTorch form per matrix: estimates, the copy, the new
+    sketches.  Tolerance: a cell sums at most a few dozen entries in 32 bits, in another order."""
+    from types import SimpleNamespace
+    from conef_b200.compressors import DenseCSHash3
+    from conef_b200.parallel.engine import sketch3_group
+
+    lib = native.lib()
+    gen = torch.Generator().manual_seed(23)
+    mats, comps, off = [], {}, 3
+    for k, (n, d) in enumerate(shapes):
+        mats.append(SimpleNamespace(n=n, m=d, g_off=off, numel=n * d))
+        comps[k] = DenseCSHash3(n, d, size, device=DEV, seed=5)
+        for cs in comps[k]._rows():
+            cs.copy_(torch.randn(cs.shape, generator=gen))
+        off += n * d + 1
+    work = torch.randn(off, generator=gen).to(DEV)
+    after = torch.randn(off, generator=gen).to(DEV)
+    before = torch.full_like(work, 9.0)
+    start = work.clone()
+    want = [[cs.clone() for cs in comps[k]._rows()] for k in comps]
+    group = sketch3_group(comps, mats, work)
+    assert group is not None
+    native.check(lib.conef_sketch3_query_group(work.data_ptr(), before.data_ptr(), group, len(mats), 0.3, _st()))
+    touched = torch.zeros(off, dtype=torch.bool, device=DEV)
+    for k, e in enumerate(mats):
+        sl = slice(e.g_off, e.g_off + e.numel)
+        touched[sl] = True
+        tabs = [(t[0], t[1]) for t in comps[k]._tables()]
+        est = start[sl].clone().view(e.n, e.m)
+        ref.sketch3_query_ref(est, want[k], tabs, 0.3)
+        torch.testing.assert_close(work[sl].view(e.n, e.m), est, rtol=1e-6, atol=1e-6)
+        ref.sketch3_update_ref((est - after[sl].view(e.n, e.m)), want[k], tabs, 0.7)
+    assert torch.equal(before[touched], work[touched]) and torch.equal(work[~touched], start[~touched])
+    assert bool((before[~touched] == 9.0).all())
+    native.check(lib.conef_sketch3_update_group(before.data_ptr(), after.data_ptr(), group, len(mats), 0.7, _st()))
+    for k in comps:
+        for got, w in zip(comps[k]._rows(), want[k]):
+            torch.testing.assert_close(got, w, rtol=2e-5, atol=2e-5)
+    comps[0].cs1 = comps[0].cs1.double()      # a store in another form goes through the general path
+    assert sketch3_group(comps, mats, work) is None
