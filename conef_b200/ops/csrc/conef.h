@@ -261,6 +261,8 @@ int conef_gather_segments(const ConefSeg* segs, int nsegs, const float* bucket,
 int conef_scatter_segments(const ConefSeg* segs, int nsegs, float* bucket,
                            const float* const* peer_staging, int world, const float* local_staging,
                            float scale, float* dense_err, long long total, cudaStream_t stream);
+// blks[i].start = starts[i] (host array, read before the call returns) for i < n, in stream order.
+int conef_randblock_starts(ConefBlk* blks, const long long* starts, int n, cudaStream_t stream);
 // Count-sketch mode: the first nblk_tiles tiles belong to tensors on the block layout of the hash
 // (cb_off >= 0) and are chunks of eight (block of 8 rows, cell block) units; the others are
 // (tensor, block of rows_per_cta rows).

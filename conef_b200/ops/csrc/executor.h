@@ -107,7 +107,7 @@ typedef struct ConefPsgdPlan {
 // ---- random-block family ---------------------------------------------------------------------------
 typedef struct ConefRandblockPlan {
   // static
-  const ConefBlk* blks;  int nblks, rows_per_cta;      // the block table is re-uploaded every step (new offsets)
+  const ConefBlk* blks;  int nblks, rows_per_cta;      // the table's `start` fields change every step
   ConefTileList tiles;
   const ConefSeg* segs;  int nsegs, ef_mode;
   long long total_unc, total_block;

@@ -146,6 +146,7 @@ _SIGNATURES = {
     "conef_sketch_query": ([vp, vp, C.c_int, vp, C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
     "conef_sketch_update": ([vp, vp, C.c_int, vp, vp, C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
     "conef_sketch3_query": ([vp] * 7 + [C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
+    "conef_randblock_starts": ([vp, vp, C.c_int, vp], C.c_int),
     "conef_sketch3_update": ([vp] * 7 + [C.c_int, C.c_int, C.c_int, C.c_float, vp], C.c_int),
     "conef_sketch3_query_group": ([vp] * 3 + [C.c_int, C.c_float, vp], C.c_int),
     "conef_sketch3_update_group": ([vp] * 3 + [C.c_int, C.c_float, vp], C.c_int),

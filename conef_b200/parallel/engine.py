@@ -1082,12 +1082,8 @@ class RandBlockEngine(_EngineBase):
         for k, s in enumerate(plan.segs):
             segs[k] = (s.g_off, s.dst_off, s.numel)
         self.segs_dev = native.upload_struct_array(segs, dev) if len(segs) else None
-        self.blks_dev = torch.empty(max(blks.nbytes, 1), dtype=torch.uint8, device=dev)
-        # two pinned staging copies of the block table (the block offsets change every step); an
-        # event per copy says when its upload has been consumed
-        self._pin = [torch.empty(max(blks.nbytes, 1), dtype=torch.uint8).pin_memory() for _ in range(2)] \
-            if dev.type == "cuda" else None
-        self._pin_evt = [None, None]
+        self.blks_dev = native.upload_struct_array(blks, dev) if len(blks) else None
+        self._starts = (ctypes.c_longlong * max(len(blks), 1))()      # this step's block offsets
         self.staging_unc = torch.empty(max(plan.total_unc, 1), device=dev, dtype=torch.float32)
         self.staging_blk = torch.empty(max(plan.total_block, 1), device=dev, dtype=torch.float32)
         self.err_arena = self.codes = self.scales = None
@@ -1210,19 +1206,17 @@ class RandBlockEngine(_EngineBase):
             self.bind_state(state, bidx)
         nb = len(plan.blocks)
         # shared-RNG block offsets: one draw per compressed tensor, in bucket order
-        blks = self.blks_host
-        for k, b in enumerate(plan.blocks):
-            blks["start"][k] = int(state.rng.choice(b.numel))
+        # (RandomState.choice(n) is randint(0, n) behind argument handling that takes three times as long)
+        rng, starts = state.rng, self._starts
+        if type(rng) is np.random.RandomState:
+            for k, b in enumerate(plan.blocks):
+                starts[k] = rng.randint(0, b.numel)
+        else:
+            for k, b in enumerate(plan.blocks):
+                starts[k] = int(rng.choice(b.numel))
         if nb:
-            k = self.step & 1
-            if self._pin_evt[k] is not None:
-                self._pin_evt[k].synchronize()          # the upload of two steps ago (long done)
-            raw = blks.view(np.uint8).reshape(-1)
-            self._pin[k].numpy()[: raw.size] = raw
-            self.blks_dev[: raw.size].copy_(self._pin[k][: raw.size], non_blocking=True)
-            if self._pin_evt[k] is None:
-                self._pin_evt[k] = torch.cuda.Event()
-            self._pin_evt[k].record()
+            native.check(lib.conef_randblock_starts(self.blks_dev.data_ptr(), starts, nb, st), "randblock_starts")
+            native.launch_count += 1
         symm, slot = self.symm, self.step & 1
         fused = self.slots is not None and os.environ.get("CONEF_FUSED", "1") == "1"
         holder = self.slots if fused else symm

@@ -724,3 +724,16 @@ def test_grouped_sketch3_matches_reference(shapes, size):
             torch.testing.assert_close(got, w, rtol=2e-5, atol=2e-5)
     comps[0].cs1 = comps[0].cs1.double()      # a store in another form goes through the general path
     assert sketch3_group(comps, mats, work) is None
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 600])
+def test_randblock_starts(n):
+    """Block offsets written into the table on the device, at and around the number one launch carries."""
+    blks = np.zeros(n + 1, dtype=native.BLK_DTYPE)
+    blks["numel"], blks["start"] = np.arange(n + 1) + 7, -5
+    dev = native.upload_struct_array(blks, torch.device(DEV))
+    starts = [(1 << 33) + 3 * i for i in range(n)]
+    native.check(native.lib().conef_randblock_starts(dev.data_ptr(), (C.c_longlong * n)(*starts), n, _st()))
+    got = dev.cpu().numpy().view(native.BLK_DTYPE)
+    assert got["start"].tolist() == starts + [-5]
+    assert np.array_equal(got["numel"], blks["numel"])
