@@ -346,6 +346,59 @@ __device__ __forceinline__ void apply_factor(const float (&x)[RP], const float (
   }
 }
 
+constexpr int orth_part_cols(int rp) { return rp * rp < 32 ? 32 : rp * rp > 256 ? 256 : rp * rp; }
+
+// Gram partial of a CTA's rows into out[RP x RP], fixed summation order: warps over row slices, then warps in order.
+// A warp covers the whole RP x RP matrix at once: each lane E neighbouring entries of one row of it, or, where the
+// matrix has fewer than 32 entries, the lanes take turns over the rows in NSUB groups.  One entry per lane and as
+// many passes over the rows as that takes: 1,300 cycles at 8 x 64 rows, 2,500 at 4 x 720.
+// Columns r .. RP - 1 of the rows are not initialised; nothing reads their entries.
+template <int RP>
+__device__ __forceinline__ void gram_partial(const float* xs, int rows, int r,
+                                             float (*part)[orth_part_cols(RP)], float* out) {
+  constexpr int S = RP + 1, PAIRS = RP * RP;
+  if (PAIRS <= 256) {
+    constexpr int E = PAIRS > 32 ? PAIRS / 32 : 1;
+    constexpr int NSUB = PAIRS < 32 ? 32 / PAIRS : 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per = (rows + (OC_THREADS / 32) - 1) / (OC_THREADS / 32);
+    const int i0 = warp * per, i1 = min(rows, i0 + per);
+    const int sub = lane / (32 / NSUB), e0 = (lane % (32 / NSUB)) * E;
+    const float* xa = xs + e0 / RP;
+    const float* xb = xs + e0 % RP;
+    float acc[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) acc[q] = 0.f;
+#pragma unroll 4
+    for (int i = i0 + sub; i < i1; i += NSUB) {
+      const float va = xa[i * S];
+#pragma unroll
+      for (int q = 0; q < E; ++q) acc[q] = fmaf(va, xb[i * S + q], acc[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+#pragma unroll
+      for (int o = 32 / NSUB; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+      if (sub == 0) part[warp][e0 + q] = acc[q];
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < PAIRS) {
+      float sum = 0.f;
+#pragma unroll
+      for (int w = 0; w < OC_THREADS / 32; ++w) sum += part[w][threadIdx.x];
+      out[threadIdx.x] = sum;
+    }
+  } else {
+    for (int pr = threadIdx.x; pr < PAIRS; pr += OC_THREADS) {
+      const int ca = pr / RP, cb = pr % RP;
+      float acc = 0.f;
+      if (ca < r && cb < r)
+        for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
+      out[pr] = acc;
+    }
+  }
+}
+
 template <int RP>
 __global__ void __launch_bounds__(OC_THREADS, RP <= 16 ? 2 : 1)
 k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, int ntiles, int which,
@@ -356,7 +409,7 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
   extern __shared__ float xs[];                    // OC_ROWS x (RP + 1): the chunk's rows
   constexpr int S = RP + 1;
   __shared__ float G[RP][RP + 1], R[RP][RP + 1], rd[RP];
-  __shared__ float part[OC_THREADS / 32][RP * RP < 32 ? 32 : RP * RP > 256 ? 256 : RP * RP];
+  __shared__ float part[OC_THREADS / 32][orth_part_cols(RP)];
   __shared__ int ok;
   bool peers_ok = true;
   if (world > 1) {
@@ -402,14 +455,16 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
   float* a = buf + off;
   // ---- load the chunk (summing the peers' copies), four loads per thread (times the peers) in flight ----
   const int nel = rows * r;
-  const bool vec4 = peer_bufs == nullptr && (r & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
+  const bool local = peer_bufs == nullptr || world <= 1;      // one rank: its slot buffer is an input like any other
+  const float* src = peer_bufs != nullptr && world <= 1 ? peer_bufs[0] + off : a;
+  const bool vec4 = local && (r & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
   if (vec4) {      // 16-byte loads of this GPU's own rows: an element group never straddles a row
     for (int q0 = 0; q0 < (nel >> 2); q0 += 4 * OC_THREADS) {
       float4 v4[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int q = q0 + u * OC_THREADS + threadIdx.x;
-        if (q < (nel >> 2)) v4[u] = __ldcg(reinterpret_cast<const float4*>(a) + q);
+        if (q < (nel >> 2)) v4[u] = __ldcg(reinterpret_cast<const float4*>(src) + q);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -429,10 +484,10 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
       const int i = base + u * OC_THREADS + threadIdx.x;
       v[u] = 0.f;
       if (i < nel) {
-        if (peer_bufs != nullptr) {
+        if (!local) {
           if (peers_ok) for (int p = 0; p < world; ++p) v[u] += ld_relaxed_sys_f32(peer_bufs[p] + off + i);
         } else {
-          v[u] = a[i];
+          v[u] = __ldcg(src + i);
         }
       }
     }
@@ -446,7 +501,6 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
     }
   }
   const int first = blockIdx.x - t.y, count = (rows_total + OC_ROWS - 1) / OC_ROWS;
-  const int pairs = r * r;
   float* pk = packed ? packed + (which == 0 ? M.ppk_off : M.qpk_off) : nullptr;
   const long long grow0 = (long long)t.y * OC_ROWS;
   const bool project = X.tables != nullptr && which == 1 && pk != nullptr && M.tab_off >= 0;
@@ -457,100 +511,78 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
 #pragma unroll 1
   for (int round = 0; round < 2; ++round) {
     __syncthreads();
-    // ---- Gram partial of the chunk, fixed summation order: warps over row slices, then warps 0..7 in order ----
-    {
-      float* g = gram + ((size_t)round * ntiles + blockIdx.x) * GRAM_STRIDE;
-      if (pairs <= 256) {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int per = (rows + (OC_THREADS / 32) - 1) / (OC_THREADS / 32);
-        const int i0 = warp * per, i1 = min(rows, i0 + per);
-        for (int pr = lane; pr < pairs; pr += 32) {
-          const int ca = pr / r, cb = pr - ca * r;
-          float acc = 0.f;
-          for (int i = i0; i < i1; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
-          part[warp][pr] = acc;
-        }
-        __syncthreads();
-        if ((int)threadIdx.x < pairs) {
-          float acc = 0.f;
-#pragma unroll
-          for (int w = 0; w < OC_THREADS / 32; ++w) acc += part[w][threadIdx.x];
-          g[threadIdx.x] = acc;
-        }
-      } else {
-        for (int pr = threadIdx.x; pr < pairs; pr += OC_THREADS) {
-          const int ca = pr / r, cb = pr - ca * r;
-          float acc = 0.f;
-          for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
-          g[pr] = acc;
-        }
-      }
-    }
+    gram_partial<RP>(xs, rows, r, part, gram + ((size_t)round * ntiles + blockIdx.x) * GRAM_STRIDE);
     if (!cta_group_barrier(bar, (unsigned)ntiles, ORTH_BARRIER_LIMIT) && threadIdx.x == 0)
       atomicExch(status, CONEF_STATUS_FLAG_TIMEOUT);
     // ---- the matrix's Gram matrix: partials in tile order; factor; inverse ----
     for (int i = threadIdx.x; i < RP * (RP + 1); i += OC_THREADS) (&R[0][0])[i] = 0.f;
-    for (int pr = threadIdx.x; pr < pairs; pr += OC_THREADS) {
+    // The partials of a tall block are many (60 for a 30,528-row embedding): all threads share them, NG groups that
+    // take every NG-th one, combined in order (one thread per entry, 64 of 256 threads at r = 8, needed four times
+    // the rounds of loads).  The order of the additions is fixed.  With the Gram and store loops shared with the
+    // cluster form: 38 -> 27 us for that embedding at r = 8.
+    constexpr int PAIRS = RP * RP, NG = PAIRS < OC_THREADS ? OC_THREADS / PAIRS : 1;
+    float* red = &part[0][0];
+    for (int q = threadIdx.x; q < PAIRS * NG; q += OC_THREADS) {
+      const int pr = q % PAIRS, grp = q / PAIRS;
       const float* g = gram + ((size_t)round * ntiles + first) * GRAM_STRIDE + pr;
       float acc = 0.f;
-      int c = 0;
-      for (; c + 8 <= count; c += 8) {          // eight loads in flight; the order of the additions is fixed
+      for (int c = grp; c < count; c += 8 * NG) {          // eight loads in flight
         float gv[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) gv[u] = __ldcg(g + (size_t)(c + u) * GRAM_STRIDE);
+        for (int u = 0; u < 8; ++u) gv[u] = c + u * NG < count ? __ldcg(g + (size_t)(c + u * NG) * GRAM_STRIDE) : 0.f;
 #pragma unroll
         for (int u = 0; u < 8; ++u) acc += gv[u];
       }
-      for (; c < count; ++c) acc += __ldcg(g + (size_t)c * GRAM_STRIDE);
-      G[pr / r][pr % r] = acc;
+      if (NG > 1) red[q] = acc;
+      else G[pr / RP][pr % RP] = acc;
+    }
+    if (NG > 1) {
+      __syncthreads();
+      if ((int)threadIdx.x < PAIRS) {
+        float acc = 0.f;
+#pragma unroll 4
+        for (int grp = 0; grp < NG; ++grp) acc += red[grp * PAIRS + threadIdx.x];
+        G[threadIdx.x / RP][threadIdx.x % RP] = acc;
+      }
     }
     __syncthreads();
     if (threadIdx.x < 32) chol_factor<RP>(G, R, rd, r, round == 0 ? ORTH_SHIFT : ORTH_SHIFT_FINAL, round == 0 ? eps : 0.f);
     __syncthreads();
     // ---- apply: every thread its rows ----
     for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
-      float av[RP];
+      float av[RP], yv[RP];
 #pragma unroll
       for (int k = 0; k < RP; ++k) av[k] = xs[i * S + k];
-      float psc = 0.f;
-      long long ph = 0;
-      if (round == 1 && project) {
-        const int e = tab[grow0 + i];
-        psc = unpack_sign(e) * X.alpha;
-        ph = unpack_bucket(e);
-      }
-      float yv[RP];
       apply_factor<RP>(av, R, rd, r, yv);
 #pragma unroll
-      for (int c = 0; c < RP; ++c) {
-        if (c < r) {
-          const float v = yv[c];
-          if (round == 0) {
-            xs[i * S + c] = v;
-          } else {
-            a[(size_t)i * r + c] = v;
-            if (packed) conef_pack_store(packed, M, which, grow0 + i, c, v, packed_np);
-            if (project) atomicAdd(zpk + conef_packed_offset(ph, c, packed_np), psc * v);
-          }
-        }
-      }
+      for (int c = 0; c < RP; ++c)
+        if (c < r) xs[i * S + c] = yv[c];
     }
   }
   // ---- columns that were exactly zero: fixed pseudo-random values instead (rare; not unrolled) ----
 #pragma unroll 1
   for (int c = 0; c < r; ++c) {
     if (R[c][c] > 0.f) continue;
-    for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
+    for (int i = threadIdx.x; i < rows; i += OC_THREADS) {      // the thread that wrote this row above
       float z[4];
       conef_philox_normal4(ORTH_REFILL_SEED + (unsigned long long)t.x * 64ull + (unsigned long long)which * 32ull + c,
                            (uint64_t)(grow0 + i), z);
-      const float v = z[0] * refill_scale;
-      a[(size_t)i * r + c] = v;
-      if (packed) conef_pack_store(packed, M, which, grow0 + i, c, v, packed_np);
-      if (project) {
-        const int e = tab[grow0 + i];
-        atomicAdd(zpk + conef_packed_offset(unpack_bucket(e), c, packed_np), unpack_sign(e) * X.alpha * v);
-      }
+      xs[i * S + c] = z[0] * refill_scale;
+    }
+  }
+  __syncthreads();
+  // ---- results, one element per thread: neighbouring threads write neighbouring addresses, and a block of few
+  //      rows keeps the whole CTA busy (a thread with a row of its own issued its r packed stores and r atomics
+  //      one after another: 3,900 cycles at 8 x 64 rows) ----
+#pragma unroll 2
+  for (int e = threadIdx.x; e < nel; e += OC_THREADS) {
+    const int i = e / r, c = e - i * r;
+    const float v = xs[i * S + c];
+    a[e] = v;
+    if (packed) conef_pack_store(packed, M, which, grow0 + i, c, v, packed_np);
+    if (project) {
+      const int h = tab[grow0 + i];
+      atomicAdd(zpk + conef_packed_offset(unpack_bucket(h), c, packed_np), unpack_sign(h) * X.alpha * v);
     }
   }
 }
@@ -700,50 +732,7 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
 #pragma unroll 1
   for (int round = 0; round < 2; ++round) {
     __syncthreads();
-    // ---- Gram partial of this CTA's rows, fixed summation order: warps over row slices, then warps in order.
-    //      A warp covers the whole RP x RP matrix at once: each lane E neighbouring entries of one row of it, or,
-    //      where the matrix has fewer than 32 entries, the lanes take turns over the rows in NSUB groups.  One entry
-    //      per lane and as many passes over the rows as that takes: 1,300 cycles at 8 x 64 rows, 2,500 at 4 x 720 ----
-    if (PAIRS_MAX <= 256) {
-      constexpr int E = PAIRS_MAX > 32 ? PAIRS_MAX / 32 : 1;
-      constexpr int NSUB = PAIRS_MAX < 32 ? 32 / PAIRS_MAX : 1;
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      const int per = (rows + (OC_THREADS / 32) - 1) / (OC_THREADS / 32);
-      const int i0 = warp * per, i1 = min(rows, i0 + per);
-      const int sub = lane / (32 / NSUB), e0 = (lane % (32 / NSUB)) * E;
-      const float* xa = xs + e0 / RP;
-      const float* xb = xs + e0 % RP;
-      float acc[E];
-#pragma unroll
-      for (int q = 0; q < E; ++q) acc[q] = 0.f;
-#pragma unroll 4
-      for (int i = i0 + sub; i < i1; i += NSUB) {
-        const float va = xa[i * S];
-#pragma unroll
-        for (int q = 0; q < E; ++q) acc[q] = fmaf(va, xb[i * S + q], acc[q]);
-      }
-#pragma unroll
-      for (int q = 0; q < E; ++q) {
-#pragma unroll
-        for (int o = 32 / NSUB; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-        if (sub == 0) part[warp][e0 + q] = acc[q];
-      }
-      __syncthreads();
-      if ((int)threadIdx.x < PAIRS_MAX) {
-        float sum = 0.f;
-#pragma unroll
-        for (int w = 0; w < OC_THREADS / 32; ++w) sum += part[w][threadIdx.x];
-        gpart[round][threadIdx.x] = sum;
-      }
-    } else {
-      for (int pr = threadIdx.x; pr < PAIRS_MAX; pr += OC_THREADS) {
-        const int ca = pr / RP, cb = pr % RP;
-        float acc = 0.f;
-        if (ca < r && cb < r)
-          for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
-        gpart[round][pr] = acc;
-      }
-    }
+    gram_partial<RP>(xs, rows, r, part, gpart[round]);
     cluster_sync_all();      // every CTA's partial of this round is in its shared memory
     // ---- the block's Gram matrix: the cluster's partials in rank order; factor; inverse ----
     for (int i = threadIdx.x; i < RP * (RP + 1); i += OC_THREADS) (&R[0][0])[i] = 0.f;
