@@ -9,12 +9,14 @@
 #include "common.cuh"
 
 constexpr int L_THREADS = 512;
-// All three kernels are bound by memory: 28 bytes per element are unavoidable (p, g, m, v in; p, m, v out), the
-// update direction that passes through the gradient adds 8.  A CTA takes a slice of L_SLICE elements of a chunk:
+// All kernels are bound by memory: 28 bytes per element are unavoidable (p, g, m, v in; p, m, v out), the
+// update direction that passes through the gradient adds 8.  A CTA of the two update kernels takes a slice of L_SLICE elements of a chunk:
 // with one CTA per 65,536-element chunk the four matrices and two feed-forward blocks of a BERT-large layer
 // (12.6 M elements, 192 chunks) were 1.3 CTAs per SM with one 4-byte load per array and thread in flight.  Slices
 // give ten CTAs per SM, 16-byte accesses where pointers and chunk starts are aligned, and shorter sums.
-// Measured on that layer, us: stage 1 110 -> 52 (36 bytes per element, 6.7 TB/s), stage 2 78 -> 20, norm 10 -> 9.
+// Measured on that layer, us: stage 1 110 -> 52 (36 bytes per element, 6.7 TB/s), stage 2 78 -> 20.  The norm
+// of all gradients keeps a CTA per chunk (10 us either way): with eight times the atomics on one sum the moments
+// were further from 64 bits (6.2e-8 against 5.5e-8 relative).
 constexpr int L_SLICE = 8192;
 
 struct LambSlice { long long lo, hi; };
@@ -27,12 +29,13 @@ __device__ __forceinline__ LambSlice lamb_slice(long long chunk, int chunk_elems
 }
 
 __global__ void __launch_bounds__(L_THREADS)
-k_lamb_gnorm(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems, int parts,
+k_lamb_gnorm(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems,
              float* __restrict__ norms) {
   __shared__ float scratch[33];
-  const int2 c = chunks[blockIdx.x / parts];
+  const int2 c = chunks[blockIdx.x];
   const ConefLambTensor T = tensors[c.x];
-  const LambSlice S = lamb_slice(c.y, chunk_elems, parts, blockIdx.x % parts, T.numel);
+  const long long lo = (long long)c.y * chunk_elems;
+  const LambSlice S = {lo, min(lo + (long long)chunk_elems, T.numel)};      // one CTA and one atomic per chunk
   float s = 0.f;
   long long i = S.lo;
   if (((reinterpret_cast<uintptr_t>(T.g + S.lo)) & 15) == 0) {
@@ -151,7 +154,7 @@ extern "C" int conef_lamb_step(const ConefLambTensor* tensors, int ntensors, con
   if ((long long)nchunks * parts > 0x7fffffffLL) { conef_set_error("lamb_step: %d chunks are too many", nchunks); return 2; }
   const int grid = nchunks * parts;
   if (max_grad_norm > 0.f) {
-    k_lamb_gnorm<<<grid, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, parts, norms);
+    k_lamb_gnorm<<<nchunks, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, norms);
     CONEF_CHECK_LAUNCH("k_lamb_gnorm");
   }
   float bc1 = 1.f, bc2 = 1.f;

@@ -521,7 +521,6 @@ class PowerSGDEngine(_EngineBase):
         good = [k for k in range(nrec) if self.tc_ok[k]]
         bad = [k for k in range(nrec) if not self.tc_ok[k]]
 
-        # used when no extent fits the launch into one wave of CTAs, or when one of the variables is set
         tuned = any(v in os.environ for v in ("CONEF_TC_WAVES", "CONEF_TC_MIN_K", "CONEF_TC_MAX_K"))
         waves = float(os.environ.get("CONEF_TC_WAVES", 3))
         min_k = int(os.environ.get("CONEF_TC_MIN_K", 384))
@@ -529,17 +528,21 @@ class PowerSGDEngine(_EngineBase):
 
         def split_tiles(mode):
             # mode 0 (P): output rows = n, K = m.  mode 1 (Q): output rows = m, K = n.
-            # Every tile gets about the same K extent: the shortest with which all CTAs are resident at once (two
-            # fit on an SM), or, with more output tiles than that, an equal share of the work for that many.
+            # Every tile gets about the same K extent: 384 to 1,024 where that makes one wave of CTAs (two fit on an
+            # SM) with work for every SM; otherwise the shortest with which all CTAs are resident at once, or, with
+            # more output tiles than that, an equal share of the work for that many.
             def view(k):        # (output rows, K) of record k, in its folded view when it has one
                 n_, m_, f = int(recs[k]["n"]), int(recs[k]["m"]), max(1, int(recs[k]["fold"]))
                 return (m_ * f, n_ // f) if mode else (n_ // f, m_ * f)
             dims = [view(k) for k in good]
-            klen_t = None if tuned else one_wave_extent(dims)
-            if klen_t is None:
-                work = sum(math.ceil(mn / 128) * K for mn, K in dims)
-                klen_t = work / max(1.0, (waves if tuned else 1.0) * TARGET_CTAS)
-                klen_t = int(min(max_k if tuned else 1 << 30, max(min_k, math.ceil(klen_t / 32) * 32)))
+            work = sum(math.ceil(mn / 128) * K for mn, K in dims)
+            klen_t = work / max(1.0, waves * TARGET_CTAS)
+            klen_t = int(min(max_k, max(min_k, math.ceil(klen_t / 32) * 32)))
+            ctas = sum(t * sp for t, _, sp in (split_k(mn, K, klen_t) for mn, K in dims))
+            # one CTA to two per SM: any extent measures the same (WideResNet, BERT and Transformer buckets within 0.5 us)
+            if not tuned and not 148 <= ctas <= TARGET_CTAS:
+                share = max(min_k, math.ceil(work / TARGET_CTAS / 32) * 32)
+                klen_t = one_wave_extent(dims) or share
             tiles = []
             for k, (mn, K) in zip(good, dims):
                 mblocks, klen, splits = split_k(mn, K, klen_t)
