@@ -118,8 +118,8 @@ def one_wave_extent(dims, slots: int = TARGET_CTAS, shortest: int = 128):
     are resident at once, or None when no extent does that.  All CTAs of a launch do about the same work, so a few
     more than the device holds (two per SM) cost a second round as long as the first.  Measured in us, P = M Q and
     Q = M^T P, against three waves of CTAs with extents of 384 to 1,024: one 512 x 512 matrix 8.1, 7.8 -> 4.7, 4.8
-    (20 CTAs of 128 instead of 10 of 256 to 512), 30528 x 1024 41, 42 -> 31, 26 (extent 928 instead of 384), two
-    640 x 5760 8.2, 7.8 -> 7.7, 7.8 (300 CTAs of 224 for the second product would take 10.2)."""
+    (20 CTAs of 128 instead of 10), 30528 x 1024 41, 42 -> 30, 26 (extent 960 instead of 384); 300 CTAs where 200
+    fit: 7.8 -> 10.2 (Q of two 640 x 5760)."""
     if not dims:
         return None
     longest = max(K for _, K in dims)
