@@ -14,7 +14,7 @@ constexpr int L_THREADS = 512;
 // elements of a chunk: with one CTA per 65,536-element chunk the four matrices and two feed-forward blocks of a
 // BERT-large layer (12.6 M elements, 192 chunks) were 1.3 CTAs per SM with one 4-byte load per array and thread in
 // flight.  Slices give ten CTAs per SM, 16-byte accesses where pointers and chunk starts are aligned, and shorter
-// sums.  Measured on that layer, us: stage 1 110 -> 52 (36 bytes per element, 8.6 TB/s counting what L2 serves),
+// sums.  Measured on that layer, us: stage 1 110 -> 52 (its 28 bytes per element at 6.7 TB/s, the copy rate),
 // stage 2 78 -> 20.  The norm of all gradients keeps a CTA per chunk (10 us either way): with eight times the atomics
 // on one sum the results were further from 64 bits than at one CTA per chunk (6.2e-8 against 4.9e-8 relative).
 constexpr int L_SLICE = 8192;
