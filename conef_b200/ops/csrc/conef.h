@@ -104,8 +104,9 @@ typedef struct ConefOrthExtra {
   float seg_scale;
   // which == 1 only: the last pass adds alpha * s_j * Q[j, :] to cell h_j of the sketch record's
   // small operand Z = alpha H^T Q, directly in the packed layout the tensor-core kernel reads
-  // (record nm + i describes the sketch of matrix i; `packed` must be given; the Z part of the
-  // packed buffer must be one of the zeroed regions).
+  // (record nm + i describes the sketch of matrix i; `packed` must be given).  The call clears Z
+  // itself, record by record; Z must not lie in zero0 / zero1, whose clearing is not ordered
+  // against these additions.
   float alpha;
   int nm;
   const int32_t* tables;

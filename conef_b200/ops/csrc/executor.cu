@@ -102,7 +102,7 @@ int correct(ConefPsgdPlan* plan, const ConefCorr* table, bool over_n, float* T, 
 
 // The fused pipeline: ten launches per bucket and step (plus the SIMT kernels of matrices that TMA
 // cannot address, and the top-k pruning).
-//   P:  k_gram(Q) [+ clears the sketch records' packed operand, + gathers the uncompressed tensors]
+//   P:  k_gram(Q) [+ clears the sketch records' packed operand Z, + gathers the uncompressed tensors]
 //       k_qr_apply, k_qr_apply [final pass: writes Q packed, adds alpha H^T Q into the packed Z]
 //       k_tc_skinny<P>  [last CTA publishes epoch 1 to the peers]
 //   Q:  k_gram(P) [waits for epoch 1, sums the peers' P, clears the other slot's P and Q regions,
@@ -136,7 +136,7 @@ static int run_fused(ConefPsgdPlan* plan, int phases, cudaStream_t s, const uint
     X.bar = plan->one_launch_orth ? plan->done_word + 1 : nullptr;
     X.max_rank = plan->max_rank;
     set_cluster_list(plan, plan->orth_q, plan->orth_rows_q, X);
-    if (sketch) { X.zero0 = plan->zpk; X.zero0_n = plan->zpk_n; X.tables = plan->tables; X.nm = nm; X.alpha = plan->alpha; }
+    if (sketch) { X.tables = plan->tables; X.nm = nm; X.alpha = plan->alpha; }
     if (plan->total_unc) {
       X.seg_mode = 1; X.nsegs = plan->nsegs; X.segs = plan->segs; X.seg_total = plan->total_unc;
       X.bucket = plan->work; X.dense_err = seg_err; X.staging = plan->local_stage[slot];

@@ -98,7 +98,6 @@ typedef struct ConefPsgdPlan {
   int has_slots;                 // local_* / peer_* are set (symmetric memory, or plain local buffers with
                                  //    one-entry pointer tables when world == 1); they start zeroed
   uint32_t* done_word;           // device counter of the tile kernel's finished CTAs (zero between launches)
-  float* zpk;  long long zpk_n;  // packed small operands of the sketch records inside qpk
   int one_launch_orth;           // 1: orthogonalisations as one launch with two CTA barriers (done_word[1..2])
   int wait_kernel;               // 1 (world > 1): a one-CTA kernel waits for the peers' epoch ahead of each consumer
   int orth_rows_q, orth_rows_p, orth_rows_u, pad3;   // most rows of a block in each Gram-Schmidt tile list

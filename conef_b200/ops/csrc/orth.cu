@@ -78,13 +78,26 @@ __device__ __forceinline__ int orth_find_seg(const ConefSeg* segs, int n, long l
   return lo;
 }
 
+// Clears share `part` of `parts` of record rec's packed projection block Z, into which the last pass over rec's Q
+// block adds.  Only CTAs that work on rec call this, and only before a barrier that all of rec's CTAs pass (the
+// launch boundary in the three-kernel form): clearing by any other CTA could come after rec's additions, since
+// nothing makes the blocks of a launch run at the same time.
+__device__ __forceinline__ void clear_projection(const ConefMat* __restrict__ mats, const ConefOrthExtra& X, int which,
+                                                 int rec, float* __restrict__ packed, int packed_np, int part, int parts) {
+  if (X.tables == nullptr || which != 1 || packed == nullptr || mats[rec].tab_off < 0) return;
+  const ConefMat& Z = mats[X.nm + rec];
+  float* z = packed + Z.qpk_off;
+  const long long n = (long long)((Z.m + 31) & ~31) * packed_np;
+  for (long long i = (long long)part * OC_THREADS + threadIdx.x; i < n; i += (long long)parts * OC_THREADS) z[i] = 0.f;
+}
+
 // CTAs [0, ntiles): one (matrix, 512-row chunk) each.  CTAs [ntiles, gridDim.x): the uncompressed
 // tensors of the bucket (X.seg_mode).  All CTAs share the clearing of X.zero0 / X.zero1.
 __global__ void __launch_bounds__(OC_THREADS)
 k_gram(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, int ntiles, int which,
        float* __restrict__ buf, float* __restrict__ gram, const float* const* __restrict__ peer_bufs,
        const uint32_t* __restrict__ flags, int world, uint32_t epoch, int* __restrict__ status, long long spin_limit,
-       const uint32_t* __restrict__ epoch_base, const ConefOrthExtra X) {
+       const uint32_t* __restrict__ epoch_base, float* __restrict__ packed, int packed_np, const ConefOrthExtra X) {
   __shared__ float Csm[GRAM_STRIDE];
   __shared__ float scratch[OC_THREADS];
   __shared__ int ok;
@@ -128,6 +141,7 @@ k_gram(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, int nt
   const size_t off = (which == 0 ? M.p_off : M.q_off) + (size_t)t.y * OC_ROWS * r;
   const int rows = min(OC_ROWS, rows_total - t.y * OC_ROWS);
   float* a = buf + off;
+  clear_projection(mats, X, which, t.x, packed, packed_np, t.y, (rows_total + OC_ROWS - 1) / OC_ROWS);
   if (peer_bufs != nullptr) {
     for (int i = threadIdx.x; i < rows * r; i += OC_THREADS) {
       float s = 0.f;
@@ -453,6 +467,7 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
   const size_t off = (which == 0 ? M.p_off : M.q_off) + (size_t)t.y * OC_ROWS * r;
   const int rows = min(OC_ROWS, rows_total - t.y * OC_ROWS);
   float* a = buf + off;
+  clear_projection(mats, X, which, t.x, packed, packed_np, t.y, (rows_total + OC_ROWS - 1) / OC_ROWS);
   // ---- load the chunk (summing the peers' copies), four loads per thread (times the peers) in flight ----
   const int nel = rows * r;
   const bool local = peer_bufs == nullptr || world <= 1;      // one rank: its slot buffer is an input like any other
@@ -675,6 +690,7 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
   const int rows = max(0, min(rows_per, rows_total - (int)grow0));
   const size_t off = (which == 0 ? M.p_off : M.q_off) + (size_t)grow0 * r;
   float* a = buf + off;
+  clear_projection(mats, X, which, rec, packed, packed_np, (int)rank, OCL);
   // ---- load this CTA's rows (summing the peers' copies), four loads per thread (times the peers) in flight:
   //      one at a time, the 11 KB of a 720 x 4 block took 7 us ----
   const int nel = rows * r;
@@ -926,7 +942,7 @@ extern "C" int conef_orthogonalize_fused(const ConefMat* mats, const int2* tiles
   if (grid == 0) grid = 1;      // only regions to clear (after the flag wait)
   float* gram2 = gram + (size_t)ntiles * GRAM_STRIDE;
   k_gram<<<grid, OC_THREADS, 0, stream>>>(mats, tiles, ntiles, which, buf, gram,
-                                         peer_bufs, flags, world, epoch, status, spin_limit, epoch_base, X);
+                                         peer_bufs, flags, world, epoch, status, spin_limit, epoch_base, packed, packed_np, X);
   CONEF_CHECK_LAUNCH("k_gram");
   if (ntiles <= 0) return 0;
   k_qr_apply<<<ntiles, OC_THREADS, 0, stream>>>(mats, tiles, which, buf, gram, gram2, eps, ORTH_SHIFT, nullptr, 0,

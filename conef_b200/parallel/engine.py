@@ -364,7 +364,6 @@ class PowerSGDEngine(_EngineBase):
                 mats[k]["qpk_off"], mats[k]["ppk_off"] = qpk, ppk
                 qpk += pad32(int(mats[k]["m"])) * self.np_cols
                 ppk += pad32(int(mats[k]["n"])) * self.np_cols
-        self.zpk_off = qpk         # the sketch records' packed operands follow the Q blocks'
         if self.fused_err:
             for k in range(nm):
                 err = mats[nm + k]
@@ -790,8 +789,6 @@ class PowerSGDEngine(_EngineBase):
         P.fused = int(self.fused)
         P.one_launch_orth = int(os.environ.get("CONEF_ORTH_ONE", "1") == "1")
         P.wait_kernel = int(os.environ.get("CONEF_WAIT_KERNEL", "1") == "1")
-        if self.ef_mode == native.EF_SKETCH and self.qpk is not None:
-            P.zpk, P.zpk_n = ptr(self.qpk) + 4 * self.zpk_off, self.qpk_total - self.zpk_off
         self.exec_plan = P
 
     def _release_exec(self) -> None:

@@ -737,3 +737,84 @@ def test_randblock_starts(n):
     got = dev.cpu().numpy().view(native.BLK_DTYPE)
     assert got["start"].tolist() == starts + [-5]
     assert np.array_equal(got["numel"], blks["numel"])
+
+
+def _packed_offset(rows, cols, np_cols):
+    """Offsets of the packed small operand (csrc/common.cuh:conef_packed_offset) as a (rows, cols) index array."""
+    k, n = np.arange(rows)[:, None], np.arange(cols)[None, :]
+    return (k >> 3) * (np_cols * 8) + (n >> 3) * 64 + ((k & 7) >> 2) * 32 + (n & 7) * 4 + (k & 3)
+
+
+@pytest.mark.parametrize("form,count,r", [("cluster", 300, 4), ("cluster", 150, 32), ("one_launch", 100, 8),
+                                          ("one_launch", 100, 32), ("three", 300, 16)])
+def test_projection_starts_from_zero_in_every_block(form, count, r):
+    """Z = alpha H^T Q of a launch with far more thread-block clusters than the device holds at once (and, in the
+    one-launch form, spare CTAs that carry the uncompressed tensors): every block of Z is cleared before its own
+    projection is added, whatever the blocks that start later do.  Z holds garbage on entry, twice in a row.
+    Tolerance: 32-bit sums of at most a few dozen entries of unit columns, and the factorisation's own error."""
+    lib = native.lib()
+    np_cols = 16 if r <= 16 else 32
+    gen = torch.Generator().manual_seed(r)
+    shapes = [(40 + 13 * (k % 50), 8 + k % 40) for k in range(count)]        # (rows of Q, cells)
+    if form == "one_launch":
+        shapes = [(640 + m, w) for m, w in shapes[: count // 2]]             # two chunks per block, all resident
+    elif r == 32:
+        shapes = [(m + 3000, w) for m, w in shapes]                          # 50 KB of rows per CTA
+    nm = len(shapes)
+    mats = np.zeros(2 * nm, dtype=native.MAT_DTYPE)
+    q_off = qpk = tab_off = 0
+    pad32 = lambda x: (x + 31) // 32 * 32
+    blocks, tables, tiles = [], [], []
+    for k, (m, w) in enumerate(shapes):
+        mats[k]["n"], mats[k]["m"], mats[k]["r"], mats[k]["q_off"] = 1, m, r, q_off
+        mats[k]["tab_off"], mats[k]["qpk_off"], mats[k]["fold"] = tab_off, qpk, 1
+        blocks.append(torch.randn(m, r, generator=gen))
+        tables.append(torch.from_numpy(ref.packed_hash_table(m, w, 994443, 609478, layout="element").copy()))
+        tiles += [(k, c) for c in range((m + 511) // 512)]
+        q_off, tab_off, qpk = q_off + m * r, tab_off + m, qpk + pad32(m) * np_cols
+    for k, (m, w) in enumerate(shapes):
+        mats[nm + k]["n"], mats[nm + k]["m"], mats[nm + k]["r"] = 1, w, r
+        mats[nm + k]["qpk_off"], mats[nm + k]["tab_off"] = qpk, -1
+        qpk += pad32(w) * np_cols
+    md = native.upload_struct_array(mats, torch.device(DEV))
+    td = torch.tensor(tiles + [(k, m) for k, (m, _) in enumerate(shapes)], dtype=torch.int32, device=DEV)
+    tab = torch.cat(tables).to(DEV)
+    gram = torch.zeros(2 * len(tiles) * 1024, device=DEV)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    bar = torch.zeros(2, dtype=torch.int32, device=DEV)
+    packed = torch.full((qpk,), 7.0, device=DEV)
+    bucket = torch.randn(5000, generator=gen).to(DEV)
+    staging = torch.zeros_like(bucket)
+    seg = np.zeros(1, dtype=native.SEG_DTYPE)
+    seg[0] = (0, 0, bucket.numel())
+    segd = native.upload_struct_array(seg, torch.device(DEV))
+    extra = native.OrthExtra()
+    extra.max_rank, extra.alpha, extra.nm, extra.tables = r, 0.5, nm, tab.data_ptr()
+    extra.seg_mode, extra.nsegs, extra.segs, extra.seg_total = 1, 1, segd.data_ptr(), bucket.numel()
+    extra.bucket, extra.staging = bucket.data_ptr(), staging.data_ptr()
+    if form == "cluster":
+        extra.cl_list, extra.cl_nmat = td.data_ptr() + 8 * len(tiles), nm
+        extra.cl_max_rows = max(m for m, _ in shapes)
+    elif form == "one_launch":
+        extra.bar = bar.data_ptr()
+    for _ in range(2):
+        dev = torch.cat([b.reshape(-1) for b in blocks]).to(DEV)
+        native.check(lib.conef_orthogonalize_fused(md.data_ptr(), td.data_ptr(), len(tiles), 1, dev.data_ptr(), 0.0, 0, 0, 1,
+                                                   0, status.data_ptr(), 0, packed.data_ptr(), np_cols, gram.data_ptr(), 0,
+                                                   C.byref(extra), _st()))
+        torch.cuda.synchronize()
+        assert lib.conef_orth_last_launches() == (3 if form == "three" else 1) and int(status[0]) == 0
+        assert torch.equal(staging, bucket)
+        pk, q = packed.cpu().double(), dev.cpu().double()
+        at = 0
+        for k, (m, w) in enumerate(shapes):
+            qk = q[at : at + m * r].view(m, r)
+            at += m * r
+            e = tables[k].numpy().view(np.uint32)
+            sign = torch.from_numpy(np.where(e >> 31, 1.0, -1.0))
+            cell = torch.from_numpy((e & 0x7FFFFFFF).astype(np.int64))
+            want = torch.zeros(w, r, dtype=torch.float64).index_add_(0, cell, 0.5 * sign[:, None] * qk)
+            got = pk[int(mats[nm + k]["qpk_off"]) + torch.from_numpy(_packed_offset(w, r, np_cols))]
+            torch.testing.assert_close(got, want, rtol=0, atol=1e-5)
+            if m >= r:
+                torch.testing.assert_close(qk.t() @ qk, torch.eye(r, dtype=torch.float64), rtol=0, atol=1e-3)
