@@ -94,8 +94,14 @@ class FusedLAMB(Optimizer):
         entries = [(p, g["weight_decay"]) for g in self.param_groups for p in g["params"] if p.grad is not None]
         params = [p for p, _ in entries]
         for p in params:
-            self._init_state(p)
-        key = tuple((p.data_ptr(), p.grad.data_ptr(), wd) for p, wd in entries)
+            st = self._init_state(p)
+            for name in ("exp_avg", "exp_avg_sq"):      # a moment restored in another form: re-lay it once
+                t = st[name]
+                if not (t.dtype == p.dtype and t.device == p.device and t.is_contiguous() and t.shape == p.shape):
+                    st[name] = torch.empty_like(p, memory_format=torch.contiguous_format).copy_(t)
+        # the table holds raw addresses: all of them, and the lengths, are the key
+        key = tuple((p.data_ptr(), p.grad.data_ptr(), self.state[p]["exp_avg"].data_ptr(),
+                     self.state[p]["exp_avg_sq"].data_ptr(), p.numel(), wd) for p, wd in entries)
         tab = self._tables.get("all")
         if tab is None or tab["key"] != key:
             rec = np.zeros(len(params), dtype=native.LAMB_DTYPE)

@@ -818,3 +818,50 @@ def test_projection_starts_from_zero_in_every_block(form, count, r):
             torch.testing.assert_close(got, want, rtol=0, atol=1e-5)
             if m >= r:
                 torch.testing.assert_close(qk.t() @ qk, torch.eye(r, dtype=torch.float64), rtol=0, atol=1e-3)
+
+
+def _lamb_case(sizes, seed, **kw):
+    """Parameters with gradients, their optimizer after one step, and a function that gives the next step in 64 bits
+    from given moments and new gradients."""
+    from conef_b200.optim import FusedLAMB
+
+    gen = torch.Generator().manual_seed(seed)
+    params = [torch.nn.Parameter(torch.randn(n, generator=gen).to(DEV)) for n in sizes]
+    opt = FusedLAMB(params, lr=1e-2, weight_decay=0.01, max_grad_norm=0.0, **kw)
+    for p in params:
+        p.grad = torch.randn(p.numel(), generator=gen).to(DEV)
+    opt.step()
+    return params, opt, gen
+
+
+@pytest.mark.parametrize("how", ["load_state_dict", "replace", "other_form"])
+def test_lamb_uses_the_moments_of_the_state(how):
+    """Moments that were loaded or replaced between two steps (parameters and gradients stay where they are) are the
+    ones the next step reads and writes, and the tensors they replaced are left alone.  Tolerance as for the slices."""
+    import copy
+
+    params, opt, gen = _lamb_case([5, 8193, 70_001], 3)
+    old = [(opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"]) for p in params]
+    moments = [(torch.randn(p.numel(), generator=gen).to(DEV), torch.rand(p.numel(), generator=gen).to(DEV)) for p in params]
+    if how == "load_state_dict":
+        sd = copy.deepcopy(opt.state_dict())
+        for k, (m, v) in enumerate(moments):
+            sd["state"][k].update(exp_avg=m.clone(), exp_avg_sq=v.clone())
+        opt.load_state_dict(sd)
+    else:
+        for p, (m, v) in zip(params, moments):
+            if how == "other_form":      # every second element of a longer tensor, and 64 bits
+                m, v = torch.stack([m, m], 1)[:, 0], v.double()
+            opt.state[p].update(exp_avg=m.clone() if how == "replace" else m, exp_avg_sq=v.clone())
+    before = [(m.clone(), v.clone()) for m, v in old]
+    start = [p.detach().clone() for p in params]
+    for p in params:
+        p.grad.copy_(torch.randn(p.numel(), generator=gen))
+    grads = [p.grad.clone() for p in params]
+    opt.step()
+    g = opt.param_groups[0]
+    for k, p in enumerate(params):
+        want = _exact_lamb(start[k], grads[k], *moments[k], 1e-2, *g["betas"], g["eps"], 0.01, 2, 1.0)
+        for got, w in zip((p.detach(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"]), want):
+            assert float((got.double() - w).abs().max()) <= 1e-5 * float(w.abs().max()), (how, k)
+        assert all(torch.equal(a, b) for a, b in zip(old[k], before[k]))
