@@ -360,6 +360,12 @@ int conef_lamb_step(const ConefLambTensor* tensors, int ntensors, const int2* ch
                     int chunk_elems, float* norms, float lr, float beta1, float beta2, float eps,
                     int step, int bias_correction, float grad_scale, float max_grad_norm,
                     cudaStream_t stream);
+// The same with sums whose order is fixed: every rank gets the same bits from the same inputs.  The chunks of a tensor
+// are consecutive and in order; scratch: conef_lamb_scratch_floats() floats on an 8-byte boundary.
+long long conef_lamb_scratch_floats(int nchunks);
+int conef_lamb_step_ordered(const ConefLambTensor* tensors, int ntensors, const int2* chunks, int nchunks,
+                            int chunk_elems, float* scratch, float lr, float beta1, float beta2, float eps, int step,
+                            int bias_correction, float grad_scale, float max_grad_norm, cudaStream_t stream);
 
 // Multi-tensor SGD with momentum (torch.optim.SGD semantics; weight decay per tensor from the table, `v` unused;
 // first != 0: the momentum buffers are initialised with the gradient).

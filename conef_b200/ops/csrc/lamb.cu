@@ -10,32 +10,70 @@
 
 constexpr int L_THREADS = 512;
 // All kernels are bound by memory: 28 bytes per element are unavoidable (p, g, m, v in; p, m, v out), the update
-// direction that passes through the gradient adds 8.  A CTA of the two update kernels takes a slice of L_SLICE
-// elements of a chunk: with one CTA per 65,536-element chunk the four matrices and two feed-forward blocks of a
-// BERT-large layer (12.6 M elements, 192 chunks) were 1.3 CTAs per SM with one 4-byte load per array and thread in
-// flight.  Slices give ten CTAs per SM, 16-byte accesses where pointers and chunk starts are aligned, and shorter
-// sums.  Measured on that layer, us: stage 1 110 -> 52 (its 28 bytes per element at 6.7 TB/s, the copy rate),
-// stage 2 78 -> 20.  The norm of all gradients keeps a CTA per chunk (10 us either way): with eight times the atomics
-// on one sum the results were further from 64 bits than at one CTA per chunk (6.2e-8 against 4.9e-8 relative).
-constexpr int L_SLICE = 8192;
+// direction that passes through the gradient adds 8.  With one CTA per 65,536-element chunk the four matrices and
+// two feed-forward blocks of a BERT-large layer (12.6 M elements, 192 chunks) were 1.3 CTAs per SM with one 4-byte
+// load per array and thread in flight.  L_PARTS CTAs per chunk are ten per SM, with 16-byte accesses where pointers
+// and chunk starts are aligned.  Measured on that layer, us: first update pass 110 -> 53 (28 bytes per element at
+// 6.6 TB/s, the copy rate), second 78 -> 21 (part of p and the direction still in L2), gradient norm 8; a step on
+// arrays that are not in any cache 215 -> 101.
+// Every data-parallel rank runs the step on its own copy, so the norms must not depend on the order in which CTAs
+// finish: each CTA leaves its partial sum in the scratch, and each CTA of the next kernel adds them up in the same
+// order (2 us a step on that layer against atomics in the order of arrival).  A last CTA that adds up would cost 7 us in
+// the first update pass: the fence holds every CTA back until its stores are out.  A caller without room for partials (conef_lamb_step) gets a
+// cluster per chunk and one atomic per chunk, which fixes the order for tensors of up to two chunks; the first update
+// pass then takes 62 us on that layer.  Error of the updated parameters and moments against 64 bits, relative: 4.5e-8
+// to 6.1e-8 from step to step whatever the order of the sums (the gradient norm's last bit).
+constexpr int L_PARTS = 8;      // CTAs per chunk: the portable cluster size
+
+// Without room for partials: norms = {squared norm of all gradients, then of p and u per tensor}, zeroed.
+// With it: a partial of the gradient norm per chunk, and {p, u} per CTA of the first update kernel.
+struct LambSums {
+  float* norms;
+  float* gpart;
+  float2* part;
+};
+
+// Both sums at once, to all threads, in fixed order.  One barrier: `warps` (a pair per warp) is used once in a kernel.
+__device__ __forceinline__ float2 lamb_block_sum(float a, float b, float2* warps) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = make_float2(a, b);
+  __syncthreads();
+  float2 t = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int w = 0; w < L_THREADS / 32; ++w) { t.x += warps[w].x; t.y += warps[w].y; }
+  return t;
+}
 
 struct LambSlice { long long lo, hi; };
-__device__ __forceinline__ LambSlice lamb_slice(long long chunk, int chunk_elems, int parts, int part, long long numel) {
+__device__ __forceinline__ LambSlice lamb_slice(long long chunk, int chunk_elems, int part, long long numel) {
   const long long c0 = chunk * chunk_elems, c1 = min(c0 + (long long)chunk_elems, numel);
+  const long long share = ((long long)chunk_elems + 4 * L_PARTS - 1) / (4 * L_PARTS) * 4;
   LambSlice s;
-  s.lo = min(c0 + (long long)part * L_SLICE, c1);
-  s.hi = min(s.lo + (long long)L_SLICE, c1);
+  s.lo = min(c0 + part * share, c1);
+  s.hi = min(s.lo + share, c1);
   return s;
+}
+
+__device__ __forceinline__ void lamb_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float lamb_remote(const float* local, uint32_t rank) {      // *local in another CTA of the cluster
+  uint32_t ra;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+  return v;
 }
 
 __global__ void __launch_bounds__(L_THREADS)
 k_lamb_gnorm(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems,
-             float* __restrict__ norms) {
+             const LambSums sums) {
   __shared__ float scratch[33];
   const int2 c = chunks[blockIdx.x];
   const ConefLambTensor T = tensors[c.x];
   const long long lo = (long long)c.y * chunk_elems;
-  const LambSlice S = {lo, min(lo + (long long)chunk_elems, T.numel)};      // one CTA and one atomic per chunk
+  const LambSlice S = {lo, min(lo + (long long)chunk_elems, T.numel)};      // one CTA per chunk
   float s = 0.f;
   long long i = S.lo;
   if (((reinterpret_cast<uintptr_t>(T.g + S.lo)) & 15) == 0) {
@@ -49,7 +87,9 @@ k_lamb_gnorm(const ConefLambTensor* __restrict__ tensors, const int2* __restrict
   }
   for (i += threadIdx.x; i < S.hi; i += L_THREADS) { const float g = T.g[i]; s = fmaf(g, g, s); }
   s = block_sum(s, scratch);
-  if (threadIdx.x == 0) atomicAdd(&norms[0], s);
+  if (threadIdx.x != 0) return;
+  if (sums.gpart != nullptr) sums.gpart[blockIdx.x] = s;
+  else atomicAdd(&sums.norms[0], s);
 }
 
 struct LambCoef { float beta1, beta2, eps, bc1, bc2, gmul, wd; };
@@ -69,17 +109,31 @@ __device__ __forceinline__ void lamb_element(const LambCoef& K, float p, float& 
 // The moments go through the caches marked for early eviction: nothing reads them again in this step, while
 // p and the update direction are read by the next kernel, which starts with the slices that were written last.
 __global__ void __launch_bounds__(L_THREADS, 3)
-k_lamb_stage1(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems, int parts,
-              float* __restrict__ norms, float beta1, float beta2, float eps, float bc1, float bc2,
+k_lamb_stage1(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems,
+              const LambSums sums, float beta1, float beta2, float eps, float bc1, float bc2,
               float grad_scale, float max_grad_norm) {
-  __shared__ float scratch[33];
-  const int2 c = chunks[blockIdx.x / parts];
+  __shared__ float2 warps[2][L_THREADS / 32];
+  __shared__ float mine[2];      // squared norms of p and u over this CTA's slice, read by the cluster's first CTA
+  const int2 c = chunks[blockIdx.x / L_PARTS];
   const ConefLambTensor T = tensors[c.x];
-  const LambSlice S = lamb_slice(c.y, chunk_elems, parts, blockIdx.x % parts, T.numel);
+  const int part = blockIdx.x % L_PARTS;      // the rank in the cluster, where there is one
+  const LambSlice S = lamb_slice(c.y, chunk_elems, part, T.numel);
+  if (S.lo >= S.hi && sums.part != nullptr) {      // behind the tensor's end
+    if (threadIdx.x == 0) sums.part[blockIdx.x] = make_float2(0.f, 0.f);
+    return;
+  }
   // gradient un-scaling and global-norm clipping folded into one factor
   float gmul = 1.f / grad_scale;
   if (max_grad_norm > 0.f) {
-    const float gn = sqrtf(norms[0]) * gmul;
+    float sq = 0.f;
+    if (sums.gpart != nullptr) {
+      const int nchunks = gridDim.x / L_PARTS;
+      for (int k = threadIdx.x; k < nchunks; k += L_THREADS) sq += sums.gpart[k];
+      sq = lamb_block_sum(sq, 0.f, warps[0]).x;
+    } else {
+      sq = sums.norms[0];
+    }
+    const float gn = sqrtf(sq) * gmul;
     if (gn > max_grad_norm) gmul *= max_grad_norm / gn;
   }
   const LambCoef K = {beta1, beta2, eps, bc1, bc2, gmul, T.weight_decay};
@@ -111,22 +165,56 @@ k_lamb_stage1(const ConefLambTensor* __restrict__ tensors, const int2* __restric
     T.v[i] = v;
     T.g[i] = g;
   }
-  pn = block_sum(pn, scratch);
-  un = block_sum(un, scratch);
-  if (threadIdx.x == 0) {
-    atomicAdd(&norms[1 + 2 * c.x], pn);
-    atomicAdd(&norms[2 + 2 * c.x], un);
+  const float2 t = lamb_block_sum(pn, un, warps[1]);
+  pn = t.x;
+  un = t.y;
+  if (sums.part != nullptr) {
+    if (threadIdx.x == 0) sums.part[blockIdx.x] = make_float2(pn, un);
+    return;
   }
+  if (threadIdx.x == 0) { mine[0] = pn; mine[1] = un; }
+  lamb_cluster_sync();
+  if (part == 0 && threadIdx.x < 2) {
+    float v[L_PARTS], sum = 0.f;
+#pragma unroll
+    for (int q = 0; q < L_PARTS; ++q) v[q] = lamb_remote(&mine[threadIdx.x], q);
+#pragma unroll
+    for (int q = 0; q < L_PARTS; ++q) sum += v[q];
+    atomicAdd(&sums.norms[1 + 2 * c.x + threadIdx.x], sum);
+  }
+  lamb_cluster_sync();           // no CTA leaves while its sums may still be read
 }
 
-__global__ void __launch_bounds__(L_THREADS)
-k_lamb_stage2(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems, int parts,
-              const float* __restrict__ norms, float lr) {
+__global__ void __launch_bounds__(L_THREADS, 4)
+k_lamb_stage2(const ConefLambTensor* __restrict__ tensors, const int2* __restrict__ chunks, int chunk_elems,
+              const LambSums sums, float lr) {
+  __shared__ float2 warps[L_THREADS / 32];
   const int b = gridDim.x - 1 - blockIdx.x;      // backwards: the slices stage 1 wrote last are still in L2
-  const int2 c = chunks[b / parts];
+  const int2 c = chunks[b / L_PARTS];
   const ConefLambTensor T = tensors[c.x];
-  const LambSlice S = lamb_slice(c.y, chunk_elems, parts, b % parts, T.numel);
-  const float pn = sqrtf(norms[1 + 2 * c.x]), un = sqrtf(norms[2 + 2 * c.x]);
+  const LambSlice S = lamb_slice(c.y, chunk_elems, b % L_PARTS, T.numel);
+  if (S.lo >= S.hi) return;
+  float pn = 0.f, un = 0.f;
+  if (sums.part != nullptr) {
+    // this tensor's partials, L_PARTS per chunk (a division in 64 bits would take as long as the additions)
+    const unsigned nchunks = T.numel <= 0x7fffffffLL
+                                 ? ((unsigned)T.numel + (unsigned)chunk_elems - 1u) / (unsigned)chunk_elems
+                                 : (unsigned)((T.numel + chunk_elems - 1) / chunk_elems);
+    const float2* first = sums.part + (size_t)(b / L_PARTS - c.y) * L_PARTS;
+    for (unsigned k = threadIdx.x; k < nchunks * L_PARTS; k += L_THREADS) {
+      const float2 v = first[k];
+      pn += v.x;
+      un += v.y;
+    }
+    const float2 t = lamb_block_sum(pn, un, warps);
+    pn = t.x;
+    un = t.y;
+  } else {
+    pn = sums.norms[1 + 2 * c.x];
+    un = sums.norms[2 + 2 * c.x];
+  }
+  pn = sqrtf(pn);
+  un = sqrtf(un);
   const float trust = (pn > 0.f && un > 0.f) ? pn / un : 1.f;
   const float step = lr * trust;
   long long i = S.lo;
@@ -144,17 +232,14 @@ k_lamb_stage2(const ConefLambTensor* __restrict__ tensors, const int2* __restric
   for (i += threadIdx.x; i < S.hi; i += L_THREADS) T.p[i] -= step * T.g[i];
 }
 
-extern "C" int conef_lamb_step(const ConefLambTensor* tensors, int ntensors, const int2* chunks, int nchunks,
-                               int chunk_elems, float* norms, float lr, float beta1, float beta2, float eps,
-                               int step, int bias_correction, float grad_scale, float max_grad_norm,
-                               cudaStream_t stream) {
-  if (ntensors <= 0 || nchunks <= 0) return 0;
-  CONEF_CUDA(cudaMemsetAsync(norms, 0, sizeof(float) * (size_t)(1 + 2 * ntensors), stream));
-  const int parts = chunk_elems > L_SLICE ? (chunk_elems + L_SLICE - 1) / L_SLICE : 1;
-  if ((long long)nchunks * parts > 0x7fffffffLL) { conef_set_error("lamb_step: %d chunks are too many", nchunks); return 2; }
-  const int grid = nchunks * parts;
+static int lamb_step(const ConefLambTensor* tensors, int ntensors, const int2* chunks, int nchunks, int chunk_elems,
+                     const LambSums& sums, float lr, float beta1, float beta2, float eps, int step,
+                     int bias_correction, float grad_scale, float max_grad_norm, cudaStream_t stream) {
+  if ((long long)nchunks * L_PARTS > 0x7fffffffLL) { conef_set_error("lamb_step: %d chunks are too many", nchunks); return 2; }
+  const int grid = nchunks * L_PARTS;
+  if (sums.norms != nullptr) CONEF_CUDA(cudaMemsetAsync(sums.norms, 0, sizeof(float) * (size_t)(1 + 2 * ntensors), stream));
   if (max_grad_norm > 0.f) {
-    k_lamb_gnorm<<<nchunks, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, norms);
+    k_lamb_gnorm<<<nchunks, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, sums);
     CONEF_CHECK_LAUNCH("k_lamb_gnorm");
   }
   float bc1 = 1.f, bc2 = 1.f;
@@ -162,12 +247,44 @@ extern "C" int conef_lamb_step(const ConefLambTensor* tensors, int ntensors, con
     bc1 = 1.f - powf(beta1, (float)step);
     bc2 = 1.f - powf(beta2, (float)step);
   }
-  k_lamb_stage1<<<grid, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, parts, norms, beta1, beta2, eps, bc1, bc2,
-                                                 grad_scale, max_grad_norm);
-  CONEF_CHECK_LAUNCH("k_lamb_stage1");
-  k_lamb_stage2<<<grid, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, parts, norms, lr);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(L_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = L_PARTS;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = sums.part == nullptr ? 1 : 0;
+  CONEF_CUDA(cudaLaunchKernelEx(&cfg, k_lamb_stage1, tensors, chunks, chunk_elems, sums, beta1, beta2, eps, bc1, bc2,
+                                grad_scale, max_grad_norm));
+  k_lamb_stage2<<<grid, L_THREADS, 0, stream>>>(tensors, chunks, chunk_elems, sums, lr);
   CONEF_CHECK_LAUNCH("k_lamb_stage2");
   return 0;
+}
+
+extern "C" int conef_lamb_step(const ConefLambTensor* tensors, int ntensors, const int2* chunks, int nchunks,
+                               int chunk_elems, float* norms, float lr, float beta1, float beta2, float eps,
+                               int step, int bias_correction, float grad_scale, float max_grad_norm,
+                               cudaStream_t stream) {
+  if (ntensors <= 0 || nchunks <= 0) return 0;
+  const LambSums sums = {norms, nullptr, nullptr};
+  return lamb_step(tensors, ntensors, chunks, nchunks, chunk_elems, sums, lr, beta1, beta2, eps, step, bias_correction,
+                   grad_scale, max_grad_norm, stream);
+}
+
+extern "C" long long conef_lamb_scratch_floats(int nchunks) {
+  return nchunks <= 0 ? 0 : (long long)nchunks * (1 + 2 * L_PARTS);
+}
+extern "C" int conef_lamb_step_ordered(const ConefLambTensor* tensors, int ntensors, const int2* chunks, int nchunks,
+                                       int chunk_elems, float* scratch, float lr, float beta1, float beta2, float eps,
+                                       int step, int bias_correction, float grad_scale, float max_grad_norm,
+                                       cudaStream_t stream) {
+  if (ntensors <= 0 || nchunks <= 0) return 0;
+  const LambSums sums = {nullptr, scratch + 2 * (size_t)L_PARTS * nchunks, reinterpret_cast<float2*>(scratch)};
+  return lamb_step(tensors, ntensors, chunks, nchunks, chunk_elems, sums, lr, beta1, beta2, eps, step, bias_correction,
+                   grad_scale, max_grad_norm, stream);
 }
 
 // ---------------------------------------------------------------------------

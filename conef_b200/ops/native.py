@@ -204,6 +204,9 @@ _SIGNATURES = {
     "conef_psgd_step": ([C.POINTER(PsgdPlan), vp], C.c_int),
     "conef_psgd_plan_release": ([C.POINTER(PsgdPlan)], C.c_int),
     "conef_epoch_word": ([vp, C.c_uint32, C.c_int, vp], C.c_int),
+    "conef_lamb_scratch_floats": ([C.c_int], C.c_longlong),
+    "conef_lamb_step_ordered": ([vp, C.c_int, vp, C.c_int, C.c_int, vp, C.c_float, C.c_float, C.c_float, C.c_float,
+                                 C.c_int, C.c_int, C.c_float, C.c_float, vp], C.c_int),
     "conef_lamb_step": ([vp, C.c_int, vp, C.c_int, C.c_int, vp, C.c_float, C.c_float, C.c_float, C.c_float,
                          C.c_int, C.c_int, C.c_float, C.c_float, vp], C.c_int),
     "conef_cpu_hash_table": ([vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int], None),
@@ -217,7 +220,7 @@ _OPTIONAL = {}
 # How many kernels one call of an entry point enqueues (memsets not counted);
 # everything not listed launches exactly one.  Host-only entry points launch none.
 _KERNELS_PER_CALL = {
-    "conef_lamb_step": 3, "conef_orthogonalize_packed": 3, "conef_orthogonalize_fused": 3, "conef_lowrank_correct": 2, "conef_topk_keep": 7, "conef_topk_chunk": 0, "conef_orth_last_launches": 0, "conef_psgd_run": 0, "conef_psgd_plan_size": 0, "conef_mat_size": 0, "conef_randblock_run": 0, "conef_randblock_plan_size": 0, "conef_psgd_step": 0, "conef_psgd_plan_release": 0, "conef_version": 0, "conef_tc_supported": 0, "conef_tc_encode_maps": 0, "conef_last_error": 0,
+    "conef_lamb_step": 3, "conef_lamb_step_ordered": 3, "conef_lamb_scratch_floats": 0, "conef_orthogonalize_packed": 3, "conef_orthogonalize_fused": 3, "conef_lowrank_correct": 2, "conef_topk_keep": 7, "conef_topk_chunk": 0, "conef_orth_last_launches": 0, "conef_psgd_run": 0, "conef_psgd_plan_size": 0, "conef_mat_size": 0, "conef_randblock_run": 0, "conef_randblock_plan_size": 0, "conef_psgd_step": 0, "conef_psgd_plan_release": 0, "conef_version": 0, "conef_tc_supported": 0, "conef_tc_encode_maps": 0, "conef_last_error": 0,
     "conef_ipc_get_handle": 0, "conef_ipc_open_handle": 0, "conef_ipc_close_handle": 0,
     "conef_cpu_hash_table": 0, "conef_cpu_sketch_query": 0, "conef_cpu_sketch_update": 0,
     "conef_cpu_gram_schmidt": 0,

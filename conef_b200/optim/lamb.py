@@ -7,7 +7,8 @@ decay inside the update direction, and a per-tensor trust ratio
 ``|w| / |update|``.
 
 On CUDA fp32 parameters the whole step is three grouped kernel launches over
-all tensors (``csrc/lamb.cu``); the gradient buffers are overwritten with the
+all tensors (``csrc/lamb.cu``), whose sums have a fixed order, so that replicas
+with equal inputs stay equal; the gradient buffers are overwritten with the
 update direction, as apex does.  On CPU (or other dtypes) the same math runs as
 PyTorch ops.
 """
@@ -114,16 +115,16 @@ class FusedLAMB(Optimizer):
             dev = params[0].device
             tab = {"key": key, "tensors": native.upload_struct_array(rec, dev),
                    "chunks": torch.from_numpy(np.asarray(chunks, dtype=np.int32)).to(dev),
-                   "nchunks": len(chunks), "norms": torch.zeros(1 + 2 * len(params), device=dev),
-                   "n": len(params)}
+                   "nchunks": len(chunks), "n": len(params),
+                   "scratch": torch.empty(lib.conef_lamb_scratch_floats(len(chunks)), device=dev)}
             self._tables["all"] = tab
         step = self.state[params[0]]["step"] + 1
         for p in params:
             self.state[p]["step"] = step
         group = self.param_groups[0]
         b1, b2 = group["betas"]
-        native.check(lib.conef_lamb_step(
+        native.check(lib.conef_lamb_step_ordered(
             tab["tensors"].data_ptr(), tab["n"], tab["chunks"].data_ptr(), tab["nchunks"], CHUNK,
-            tab["norms"].data_ptr(), float(group["lr"]), float(b1), float(b2), float(group["eps"]), int(step),
+            tab["scratch"].data_ptr(), float(group["lr"]), float(b1), float(b2), float(group["eps"]), int(step),
             int(bool(group["bias_correction"])), float(self.grad_scale), float(group["max_grad_norm"] or 0.0),
             native.stream_ptr(params[0].device)), "lamb_step")

@@ -827,7 +827,7 @@ def _lamb_case(sizes, seed, **kw):
 
     gen = torch.Generator().manual_seed(seed)
     params = [torch.nn.Parameter(torch.randn(n, generator=gen).to(DEV)) for n in sizes]
-    opt = FusedLAMB(params, lr=1e-2, weight_decay=0.01, max_grad_norm=0.0, **kw)
+    opt = FusedLAMB(params, lr=1e-2, weight_decay=0.01, **dict(dict(max_grad_norm=0.0), **kw))
     for p in params:
         p.grad = torch.randn(p.numel(), generator=gen).to(DEV)
     opt.step()
@@ -865,3 +865,50 @@ def test_lamb_uses_the_moments_of_the_state(how):
         for got, w in zip((p.detach(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"]), want):
             assert float((got.double() - w).abs().max()) <= 1e-5 * float(w.abs().max()), (how, k)
         assert all(torch.equal(a, b) for a, b in zip(old[k], before[k]))
+
+
+@pytest.mark.parametrize("clip", [0.0, 1.0])
+@pytest.mark.parametrize("n", [16_385, 65_536, 65_537, 131_073, 1_000_003])
+def test_lamb_norms_do_not_depend_on_the_order_of_arrival(n, clip):
+    """A step from the same state gives the same bits every time, with sums over many CTAs and with clipping."""
+    results = []
+    for _ in range(25):
+        params, _, _ = _lamb_case([7, n, 1000, n], 11, max_grad_norm=clip)
+        results.append([p.detach().clone() for p in params])
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+
+
+@pytest.mark.parametrize("chunk", [8, 100, 65536])
+def test_lamb_entry_points_agree_for_any_chunk(chunk):
+    """Both entry points with chunks that do and do not fill every CTA of a chunk, against each other: the sums differ
+    in their order only (tolerance: 32-bit sums of a few thousand squares).  The one without room for partials is
+    reproducible for tensors of up to two chunks."""
+    lib = native.lib()
+    sizes = [1, 2 * chunk, chunk + 1, 3, min(chunk, 5000), 7]
+    chunks = [(t, c) for t, n in enumerate(sizes) for c in range((n + chunk - 1) // chunk)]
+    cd = torch.tensor(chunks, dtype=torch.int32, device=DEV)
+
+    def step(ordered):
+        gen = torch.Generator().manual_seed(chunk)
+        ts = [[torch.randn(n, generator=gen).to(DEV), torch.randn(n, generator=gen).to(DEV),
+               torch.randn(n, generator=gen).to(DEV), torch.rand(n, generator=gen).to(DEV)] for n in sizes]
+        rec = np.zeros(len(sizes), dtype=native.LAMB_DTYPE)
+        for t, q in enumerate(ts):
+            rec[t] = (*(x.data_ptr() for x in q), sizes[t], 0.01, 0)
+        rd = native.upload_struct_array(rec, torch.device(DEV))
+        n = lib.conef_lamb_scratch_floats(len(chunks)) if ordered else 1 + 2 * len(sizes)
+        scratch = torch.full((n + 1,), 3.0, device=DEV)
+        fn = lib.conef_lamb_step_ordered if ordered else lib.conef_lamb_step
+        native.check(fn(rd.data_ptr(), len(sizes), cd.data_ptr(), len(chunks), chunk, scratch.data_ptr(), 1e-2, 0.9, 0.999,
+                        1e-6, 3, 1, 1.0, 0.0, _st()))
+        torch.cuda.synchronize()
+        assert float(scratch[n]) == 3.0                       # nothing behind the scratch is touched
+        return [q[0] for q in ts] + [q[2] for q in ts] + [q[3] for q in ts]
+
+    want, plain = step(True), step(False)
+    for a, b in zip(want, plain):
+        torch.testing.assert_close(a, b, rtol=2e-6, atol=2e-7)
+    for _ in range(10):
+        assert all(torch.equal(a, b) for a, b in zip(want, step(True)))
+        assert all(torch.equal(a, b) for a, b in zip(plain, step(False)))
