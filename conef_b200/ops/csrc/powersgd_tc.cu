@@ -6,15 +6,15 @@
 // for every TMA-addressable matrix of a bucket in one launch (grouped, split-K).
 //
 // One CTA computes a 128 x NP accumulator tile (NP = r padded to 16 or 32) in
-// tensor memory:
+// tensor memory, in up to eight partial accumulators:
 //   warp 4, one lane : TMA producer - per stage four 32x32 fp32 boxes of M
 //                      (cp.async.bulk.tensor.2d, 128-byte swizzle) and one bulk copy of the
 //                      matching 32 x NP slice of the small operand, which the host side keeps
 //                      pre-packed in the K-major core-matrix layout; local memory only
 //   warps 0-3        : epilogue
 //   warp 5, one lane : tcgen05.mma.kind::tf32 (4 x K=8 per stage), tcgen05.commit frees the stage
-//   epilogue         : tcgen05.ld 32 lanes x NP columns per warp -> r floats per output row,
-//                      plain store or fp32 atomics when K is split across CTAs
+//   epilogue         : tcgen05.ld 32 lanes x NP columns per warp and accumulator -> r floats per
+//                      output row, plain store or fp32 atomics when K is split across CTAs
 //   tail             : the CTA that finishes last (a device counter) publishes the bucket's epoch
 //                      in every peer's flag array (release at system scope), so the all-reduce
 //                      that consumes the product starts from this kernel, not from a launch of
@@ -38,6 +38,12 @@ constexpr int TC_STAGES = 6;
 constexpr int TC_THREADS = 192;
 constexpr int A_STAGE_BYTES = TC_BM * TC_BK * 4;   // 16 KB
 constexpr int BOX_BYTES = 32 * 32 * 4;             // one TMA box
+// The tensor core's additions into an accumulator are not rounded to nearest: their error grows with the number of
+// additions (relative error of the product of the 19-bit operands, 30,528 rows: 0.9e-6 after K = 384, 2.3e-6 after
+// 1,024, 4.8e-6 after 2,048), and it does not average out against the rounding of the operands.  So a CTA starts a
+// new accumulator every TC_ACC_ITERS stages (K = 384) while it has some left, and the epilogue adds them up in fp32.
+constexpr int TC_ACCS = 8;
+constexpr int TC_ACC_ITERS = 12;
 constexpr long long MBAR_SPIN_LIMIT = 4LL * 1000 * 1000;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -115,6 +121,15 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// 16 columns of this warp's 32 lanes; complete after tcgen05.wait::ld
+__device__ __forceinline__ void tmem_load16(uint32_t* v, uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr) : "memory");
+}
+
 struct TcSignal {           // all zero: nothing is published
   uint32_t* done;           // counter of finished CTAs; zero between launches (the last CTA resets it)
   uint32_t* const* peer_flags;
@@ -165,6 +180,7 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
   const int k_total = Q_MODE ? M.n / fold : M.m * fold;
   const int k_end = min(k_total, T.k0 + T.klen);
   const int iters = (k_end - T.k0 + TC_BK - 1) / TC_BK;
+  const int acc_iters = max(TC_ACC_ITERS, (iters + TC_ACCS - 1) / TC_ACCS);      // stages per accumulator
   // small operand, packed: per K step of 8 rows NP * 8 floats (see conef_packed_offset)
   const float* small = small_packed + (Q_MODE ? (fold > 1 ? M.ppk_fold_off : M.ppk_off) : M.qpk_off);
   float* out = out_base + (Q_MODE ? M.q_off : M.p_off);              // (mn_total x r), row-major
@@ -183,8 +199,8 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    // 32 columns of tensor memory: 128 lanes x NP fp32 accumulators
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;" ::"r"(smem_u32(tmem_slot)) : "memory");
+    // TC_ACCS accumulators of NP columns (128 lanes each): two CTAs of an SM take half of its tensor memory
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TC_ACCS * NP) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -219,8 +235,11 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
       constexpr uint32_t idesc = make_idesc(NP, Q_MODE ? 1 : 0, 0);
       constexpr uint32_t B_STEP = (NP / 8) * 256;     // bytes of the small operand per K step of 8
       bool ok = true;
+      uint32_t acc = tmem_base;      // this stage's accumulator
+      int left = acc_iters;          // stages it still takes
       for (int it = 0; it < iters && ok; ++it) {
         const int s = it % TC_STAGES;
+        if (left == 0) { acc += NP; left = acc_iters; }
         ok = mbar_wait(smem_u32(full + s), (it / TC_STAGES) & 1, abort_flag);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -235,8 +254,9 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
             da = make_smem_desc(a_addr + ks * 32, 16, 1024, 2);
           // small operand, K-major without swizzle: K-adjacent cores 128 B apart, 8-row N groups 256 B apart
           db = make_smem_desc(b_addr + ks * B_STEP, 128, 256, 0);
-          umma_tf32(tmem_base, da, db, idesc, (it > 0 || ks > 0) ? 1u : 0u);
+          umma_tf32(acc, da, db, idesc, (left < acc_iters || ks > 0) ? 1u : 0u);
         }
+        --left;
         umma_commit(smem_u32(empty + s));     // stage reusable once these MMAs have read it
       }
       if (ok) umma_commit(smem_u32(accum));   // accumulator complete
@@ -249,25 +269,18 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t v[NP];
       const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
-      if (NP == 16) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(taddr) : "memory");
-      } else {
 #pragma unroll
-        for (int half = 0; half < NP / 16; ++half) {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(v[16 * half + 0]), "=r"(v[16 * half + 1]), "=r"(v[16 * half + 2]), "=r"(v[16 * half + 3]),
-                "=r"(v[16 * half + 4]), "=r"(v[16 * half + 5]), "=r"(v[16 * half + 6]), "=r"(v[16 * half + 7]),
-                "=r"(v[16 * half + 8]), "=r"(v[16 * half + 9]), "=r"(v[16 * half + 10]), "=r"(v[16 * half + 11]),
-                "=r"(v[16 * half + 12]), "=r"(v[16 * half + 13]), "=r"(v[16 * half + 14]), "=r"(v[16 * half + 15])
-              : "r"(taddr + 16 * half) : "memory");
-        }
-      }
+      for (int half = 0; half < NP / 16; ++half) tmem_load16(v + 16 * half, taddr + 16 * half);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      const int naccs = (iters + acc_iters - 1) / acc_iters;
+      for (int q = 1; q < naccs; ++q) {
+        uint32_t w[NP];
+#pragma unroll
+        for (int half = 0; half < NP / 16; ++half) tmem_load16(w + 16 * half, taddr + q * NP + 16 * half);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < NP; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) + __uint_as_float(w[c]));
+      }
       const int row = T.mn0 + warp * 32 + lane;
       if (row < mn_total) {
         if (!Q_MODE || fold == 1) {
@@ -310,7 +323,7 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
     __syncthreads();
   }
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem_base) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TC_ACCS * NP) : "memory");
   }
   // ---------------- publish: the last CTA tells the peers that this GPU's product is complete ----------------
   if (sig.done != nullptr && threadIdx.x == 0) {

@@ -128,3 +128,31 @@ def test_hook_with_tensorcore_path_matches_cpu(single_rank_group, monkeypatch, k
     cpu = run("cpu", "torch", "0")
     for a, c in zip(tc, cpu):
         assert _rel(a, c) < 1e-2, _rel(a, c)
+
+
+@pytest.mark.parametrize("K", [64, 384, 416, 1536, 3072, 12288])
+@pytest.mark.parametrize("rank", [8, 24])
+def test_long_extents_do_not_lose_bits(single_rank_group, monkeypatch, K, rank):
+    """One CTA over the whole K range, operands that the tensor core takes exactly (19 bits), against 64 bits.  Its
+    additions are not rounded to nearest: an accumulator that takes n products of 8 loses up to n * 2^-24 of its value
+    on average.  At most 48 products go into one of the eight accumulators up to K = 3,072, K / 64 beyond."""
+    for var in ("CONEF_TC_MIN_K", "CONEF_TC_MAX_K"):
+        monkeypatch.setenv(var, str(K))
+    cut = lambda x: (x.view(torch.int32) & ~0x1FFF).view(torch.float32)
+    bound = max(min(K // 8, 48), K // 64) * 2.0 ** -24
+    for shape, mode in (((256, K), 0), ((K, 256), 1)):
+        eng, b = _engine(rank, monkeypatch, single_rank_group, [shape])
+        tiles = eng.tc_p_tiles if mode == 0 else eng.qsets["all"][0]
+        assert eng.use_tc and [int(t[3]) for t in tiles] == [K, K]
+        buf, plan = b.buffer(), eng.plan
+        buf.copy_(cut(buf))
+        e = plan.mats[0]
+        m = buf.view(e.n, e.m)
+        small = cut(torch.randn((e.m, e.n)[mode], e.r, generator=torch.Generator().manual_seed(K)).to(DEV))
+        out = torch.zeros((plan.total_p, plan.total_q)[mode], device=DEV)
+        launch = eng._launch_q if mode else eng._launch_p
+        launch(buf.data_ptr(), 0, small.reshape(-1), out, native.stream_ptr(buf.device))
+        torch.cuda.synchronize()
+        assert int(eng.status[0]) == 0
+        want = (m.double().t() if mode else m.double()) @ small.double()
+        assert _rel(out.view_as(want).double(), want) < bound + 2.0 ** -24, (K, mode)
