@@ -40,10 +40,11 @@ constexpr int A_STAGE_BYTES = TC_BM * TC_BK * 4;   // 16 KB
 constexpr int BOX_BYTES = 32 * 32 * 4;             // one TMA box
 // The tensor core's additions into an accumulator are not rounded to nearest: their error grows with the number of
 // additions (relative error of the product of the 19-bit operands, 30,528 rows: 0.9e-6 after K = 384, 2.3e-6 after
-// 1,024, 4.8e-6 after 2,048), and it does not average out against the rounding of the operands.  So a CTA starts a
-// new accumulator every TC_ACC_ITERS stages (K = 384) while it has some left, and the epilogue adds them up in fp32.
+// 1,024, 4.8e-6 after 2,048), and it does not average out against the rounding of the operands.  So a CTA with more
+// than TC_ONE_ACC_ITERS stages (K = 512, 1.2e-6) starts a new accumulator every TC_ACC_ITERS (K = 384) while it has
+// some left, and the epilogue adds them up in fp32.
 constexpr int TC_ACCS = 8;
-constexpr int TC_ACC_ITERS = 12;
+constexpr int TC_ONE_ACC_ITERS = 16, TC_ACC_ITERS = 12;
 constexpr long long MBAR_SPIN_LIMIT = 4LL * 1000 * 1000;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -180,7 +181,8 @@ k_tc_skinny(const ConefMat* __restrict__ mats, const CUtensorMap* __restrict__ m
   const int k_total = Q_MODE ? M.n / fold : M.m * fold;
   const int k_end = min(k_total, T.k0 + T.klen);
   const int iters = (k_end - T.k0 + TC_BK - 1) / TC_BK;
-  const int acc_iters = max(TC_ACC_ITERS, (iters + TC_ACCS - 1) / TC_ACCS);      // stages per accumulator
+  const int acc_iters = iters <= TC_ONE_ACC_ITERS ? TC_ONE_ACC_ITERS
+                                                  : max(TC_ACC_ITERS, (iters + TC_ACCS - 1) / TC_ACCS);
   // small operand, packed: per K step of 8 rows NP * 8 floats (see conef_packed_offset)
   const float* small = small_packed + (Q_MODE ? (fold > 1 ? M.ppk_fold_off : M.ppk_off) : M.qpk_off);
   float* out = out_base + (Q_MODE ? M.q_off : M.p_off);              // (mn_total x r), row-major

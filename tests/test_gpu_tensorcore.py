@@ -130,16 +130,16 @@ def test_hook_with_tensorcore_path_matches_cpu(single_rank_group, monkeypatch, k
         assert _rel(a, c) < 1e-2, _rel(a, c)
 
 
-@pytest.mark.parametrize("K", [64, 384, 416, 1536, 3072, 12288])
+@pytest.mark.parametrize("K", [64, 384, 512, 544, 1536, 3072, 12288])
 @pytest.mark.parametrize("rank", [8, 24])
 def test_long_extents_do_not_lose_bits(single_rank_group, monkeypatch, K, rank):
     """One CTA over the whole K range, operands that the tensor core takes exactly (19 bits), against 64 bits.  Its
     additions are not rounded to nearest: an accumulator that takes n products of 8 loses up to n * 2^-24 of its value
-    on average.  At most 48 products go into one of the eight accumulators up to K = 3,072, K / 64 beyond."""
+    on average.  One accumulator takes K / 8 products up to K = 512; beyond, each of eight takes 48, or K / 64."""
     for var in ("CONEF_TC_MIN_K", "CONEF_TC_MAX_K"):
         monkeypatch.setenv(var, str(K))
     cut = lambda x: (x.view(torch.int32) & ~0x1FFF).view(torch.float32)
-    bound = max(min(K // 8, 48), K // 64) * 2.0 ** -24
+    bound = (K // 8 if K <= 512 else max(48, K // 64)) * 2.0 ** -24
     for shape, mode in (((256, K), 0), ((K, 256), 1)):
         eng, b = _engine(rank, monkeypatch, single_rank_group, [shape])
         tiles = eng.tc_p_tiles if mode == 0 else eng.qsets["all"][0]
