@@ -115,11 +115,7 @@ def split_k(mn: int, K: int, extent: int):
 
 def one_wave_extent(dims, slots: int = TARGET_CTAS, shortest: int = 128):
     """The shortest K extent (a multiple of 32) at which the tensor-core tiles of all (mn, K) products of a launch
-    are resident at once, or None when no extent does that.  All CTAs of a launch do about the same work, so a few
-    more than the device holds (two per SM) cost a second round as long as the first.  Measured in us, P = M Q and
-    Q = M^T P, against three waves of CTAs with extents of 384 to 1,024: one 512 x 512 matrix 8.1, 7.8 -> 4.7, 4.8
-    (20 CTAs of 128 instead of 10), 30528 x 1024 41, 42 -> 30, 26 (extent 960 instead of 384); 300 CTAs where 200
-    fit: 7.8 -> 10.2 (Q of two 640 x 5760)."""
+    are resident at once, or None when no extent does that."""
     if not dims:
         return None
     longest = max(K for _, K in dims)
@@ -132,6 +128,86 @@ def one_wave_extent(dims, slots: int = TARGET_CTAS, shortest: int = 128):
             return None
         extent += max(32, extent // 512 * 32)
     return None
+
+
+LARGE_LAUNCH = 100_000_000      # bytes of operands from which a launch runs from HBM (L2 holds 126 MB)
+
+
+def product_slots(np_cols: int) -> int:
+    """Resident CTAs of a tensor-core launch: two per SM at 16 accumulator columns, one at 32 (six stages of 20 KB)."""
+    return TARGET_CTAS if np_cols <= 16 else 148
+
+
+def product_time(groups, extent: int, np_cols: int, rank: int) -> float:
+    """Modelled time in us of a tensor-core launch at a target K extent, less its constant part.
+
+    ``groups``: {products that add into one output: how many such outputs}, a product being (output rows, K, whether
+    it adds with atomics even when one CTA covers K).  A CTA costs a fixed time (prologue, drain; more per output
+    column with atomics) and, per unit of K, what a lone CTA reaches or its share of the bandwidth.  From L2, rounds of
+    CTAs follow each other and the last one shares the bandwidth among fewer.  From HBM the bandwidth decides, which
+    is best with about one CTA per SM (30528 x 1024, Q: 135 CTAs 26 us, 180 27, 216 to 297 29 to 34; six 4390 x 1216
+    with dense feedback, Q: 120 CTAs 27 us, 240 33).  CTAs that split one output add to the same addresses, one after
+    another.  Fitted to 147 launches at up to 20 extents each (64 x 576 to 38400 x 1024, ranks 1 to 32, with and
+    without error records), of which a third ran from HBM: the pick is on average 2 % slower than the best measured."""
+    slots = product_slots(np_cols)
+    n = work = longest = adds = most = nbytes = 0
+    for group, count in groups.items():
+        adders = 0
+        for mn, K, atomic in group:
+            tiles, klen, splits = split_k(mn, K, extent)
+            n += count * tiles * splits
+            work += count * tiles * splits * klen
+            nbytes += count * 4 * mn * K
+            longest = max(longest, klen)
+            adders += splits
+            if atomic or splits > 1:
+                adds += count * tiles * splits
+        most = max(most, adders)
+    columns, mean = rank * adds / n, work / n
+    if nbytes > LARGE_LAUNCH:
+        fixed = 1.1 + 0.22 * columns
+        crowd = 0.15 * min(1.0, max(0.0, (n - 148) / 35)) if slots > 148 else 0.0
+        t = max(fixed * max(1.0, n / slots) + nbytes / 6.9e6 * (1 + crowd), fixed + 0.0105 * longest)
+        if slots == 148:
+            t = max(t, math.ceil(n / slots) * (fixed + 0.009 * mean))
+    else:
+        fixed = 4.0 + 0.09 * columns
+        per_k = lambda ctas: max(0.0088, 3.4e-5 * ctas)
+        rounds, rest = divmod(n, slots)
+        t = rounds * (fixed + mean * per_k(slots)) + (fixed + mean * per_k(rest) if rest else 0.0)
+        t = max(t, fixed + longest * per_k(1)) + (0.5 if n > 148 else 0.0)      # some SMs take a second CTA
+    return (t ** 4 + (most * (0.05 + 0.02 * rank)) ** 4) ** 0.25
+
+
+def product_extent(products, base: int, np_cols: int, rank: int) -> int:
+    """K extent of the CTAs of one tensor-core launch over ``products``: (output rows, K, output, atomic).
+
+    ``base`` (three rounds of CTAs of K = 384 to 1,024) unless another extent is at least 14 % shorter by
+    ``product_time``: with that margin two of those 147 launches were slower than at ``base`` (by 3 and 4 %), with
+    10 % nine were, by up to 15 %.  Measured in us, P and Q, base -> choice: 512 x 512 at rank 4 8.4, 8.4 -> 4.9, 5.0;
+    30528 x 1024 at rank 8 33, 42 -> 29, 26, at rank 24 61, 66 -> 41, 30; two 640 x 5760 at rank 32 22, 21 -> 14, 12;
+    38400 x 1024 40, 46 -> 38, 31; five 2716 x 2016 with dense feedback 45, 44 -> 46, 41, at rank 24 70, 70 -> 56, 58."""
+    if not products:
+        return base
+    outputs = {}
+    for mn, K, out, atomic in products:
+        outputs.setdefault(out, []).append((mn, K, bool(atomic)))
+    groups = {}
+    for group in outputs.values():
+        key = tuple(sorted(group))
+        groups[key] = groups.get(key, 0) + 1
+    dims = [(mn, K) for mn, K, _, _ in products]
+    longest = max(K for _, K in dims)
+    candidates, last = [one_wave_extent(dims, product_slots(np_cols))], 0
+    for splits in range(max(1, longest // 128), 0, -1):      # every split of the longest product, 2 % apart
+        extent = math.ceil(math.ceil(longest / splits) / 32) * 32
+        if extent > 1.02 * last:
+            candidates.append(extent)
+            last = extent
+    best = min((e for e in candidates if e), key=lambda e: product_time(groups, e, np_cols, rank))
+    if product_time(groups, base, np_cols, rank) <= 1.16 * product_time(groups, best, np_cols, rank):
+        return base
+    return best
 
 
 def decompress_rows(block_ctas, off_rows: int, off_width: int) -> int:
@@ -527,9 +603,7 @@ class PowerSGDEngine(_EngineBase):
 
         def split_tiles(mode):
             # mode 0 (P): output rows = n, K = m.  mode 1 (Q): output rows = m, K = n.
-            # Every tile gets about the same K extent: 384 to 1,024 where that makes one wave of CTAs (two fit on an
-            # SM) with work for every SM; otherwise the shortest with which all CTAs are resident at once, or, with
-            # more output tiles than that, an equal share of the work for that many.
+            # Every tile gets about the same K extent: three rounds of CTAs, or what product_extent finds shorter.
             def view(k):        # (output rows, K) of record k, in its folded view when it has one
                 n_, m_, f = int(recs[k]["n"]), int(recs[k]["m"]), max(1, int(recs[k]["fold"]))
                 return (m_ * f, n_ // f) if mode else (n_ // f, m_ * f)
@@ -537,17 +611,15 @@ class PowerSGDEngine(_EngineBase):
             work = sum(math.ceil(mn / 128) * K for mn, K in dims)
             klen_t = work / max(1.0, waves * TARGET_CTAS)
             klen_t = int(min(max_k, max(min_k, math.ceil(klen_t / 32) * 32)))
-            ctas = sum(t * sp for t, _, sp in (split_k(mn, K, klen_t) for mn, K in dims))
-            # one CTA to two per SM: any extent measures the same (WideResNet, BERT and Transformer buckets within 0.5 us)
-            if not tuned and not 148 <= ctas <= TARGET_CTAS:
-                share = max(min_k, math.ceil(work / TARGET_CTAS / 32) * 32)
-                klen_t = one_wave_extent(dims) or share
+            shared = self.fused_err if mode == 0 else self.ef_mode == native.EF_DENSE      # two records, one output
+            folded = [mode == 1 and int(recs[k]["fold"]) > 1 for k in good]      # row blocks that add into one Q block
+            if not tuned:
+                klen_t = product_extent([(mn, K, k % self.nm if shared else k, shared or f)
+                                         for k, f, (mn, K) in zip(good, folded, dims)], klen_t, self.np_cols, self.max_rank)
             tiles = []
-            for k, (mn, K) in zip(good, dims):
+            for k, f, (mn, K) in zip(good, folded, dims):
                 mblocks, klen, splits = split_k(mn, K, klen_t)
-                shared = self.fused_err if mode == 0 else self.ef_mode == native.EF_DENSE
-                folded_q = mode == 1 and int(recs[k]["fold"]) > 1       # its row blocks add into one Q block
-                flag = (1 << 30) if (splits > 1 or shared or folded_q) else 0
+                flag = (1 << 30) if (splits > 1 or shared or f) else 0
                 for mb in range(mblocks):
                     for sp in range(splits):
                         tiles.append((k | flag, mb * 128, sp * klen, klen))

@@ -1,9 +1,11 @@
 """Rules that size the launches of a bucket's plan (host side only)."""
 import math
+import random
 
 import pytest
 
-from conef_b200.parallel.engine import decompress_rows, one_wave_extent, split_k
+from conef_b200.parallel.engine import (decompress_rows, one_wave_extent, product_extent, product_slots, product_time,
+                                        split_k)
 
 
 def _block_ctas(shapes):
@@ -43,3 +45,95 @@ def test_one_wave_extent_gives_up_on_too_many_output_tiles():
     assert one_wave_extent([]) is None
     assert one_wave_extent([(128 * 297, 64)]) is None
     assert one_wave_extent([(30528, 1024), (30528, 104)]) is None
+
+
+def _base_extent(dims):
+    """The plan's starting point: three rounds of CTAs, K = 384 to 1,024."""
+    work = sum(math.ceil(mn / 128) * K for mn, K in dims)
+    return int(min(1024, max(384, math.ceil(work / (3 * 296) / 32) * 32)))
+
+
+def _products(shapes, mode, err, width=0.1):
+    """Products of one launch: per (n, m) the gradient's and, for dense feedback or the sketch, the error record's."""
+    out = []
+    for k, (n, m) in enumerate(shapes):
+        records = [(n, m)] + {"dense": [(n, m)], "sketch": [(n, max(4, int(m * width) // 4 * 4))], "none": []}[err]
+        for i, (rows, cols) in enumerate(records):
+            shared = err == "dense" or (err == "sketch" and mode == 0)
+            out.append((cols, rows, k if shared else (k, i), shared) if mode else (rows, cols, k if shared else (k, i), shared))
+    return out
+
+
+def _groups(products):
+    outputs, groups = {}, {}
+    for mn, K, out, atomic in products:
+        outputs.setdefault(out, []).append((mn, K, bool(atomic)))
+    for g in outputs.values():
+        groups[tuple(sorted(g))] = groups.get(tuple(sorted(g)), 0) + 1
+    return groups
+
+
+def _ctas(products, extent):
+    """(CTAs, longest K extent) of a launch."""
+    pieces = [split_k(mn, K, extent) for mn, K, _, _ in products]
+    return sum(t * s for t, _, s in pieces), max(k for _, k, _ in pieces)
+
+
+@pytest.mark.parametrize("rank", [4, 16, 24])
+@pytest.mark.parametrize("err", ["dense", "sketch", "none"])
+def test_product_extent_is_never_modelled_longer_than_the_base(rank, err):
+    """A few hundred random buckets: the launch is no longer than at the base extent by the model of its rounds, the
+    extent is a multiple of 32, and the CTAs cover K.  At 32 accumulator columns one CTA fits on an SM."""
+    rng = random.Random(rank)
+    np_cols = 16 if rank <= 16 else 32
+    for _ in range(150):
+        shapes = [(int(math.exp(rng.uniform(math.log(16), math.log(40000)))), 4 * rng.randint(8, 1024))
+                  for _ in range(rng.randint(1, 8))]
+        shapes = [s for s in shapes if s[0] * s[1] < 40_000_000] or [(512, 512)]
+        for mode in (0, 1):
+            products = _products(shapes, mode, err)
+            dims = [(mn, K) for mn, K, _, _ in products]
+            base = _base_extent(dims)
+            extent = product_extent(products, base, np_cols, rank)
+            assert extent % 32 == 0 and extent >= 32
+            for mn, K in dims:
+                tiles, klen, splits = split_k(mn, K, extent)
+                assert klen % 32 == 0 and (splits - 1) * klen < K <= splits * klen and tiles * 128 >= mn
+            groups = _groups(products)
+            assert product_time(groups, extent, np_cols, rank) <= product_time(groups, base, np_cols, rank)
+
+
+def test_product_slots():
+    """Resident CTAs per launch: two per SM at 16 accumulator columns; 32 columns need 121 KB of shared memory each."""
+    assert (product_slots(16), product_slots(32)) == (296, 148)
+
+
+@pytest.mark.parametrize("shapes,err,rank", [([(2716, 2016)] * 5, "dense", 8), ([(4392, 1216)] * 6, "dense", 8),
+                                             ([(1536, 2048)] * 7, "dense", 4), ([(38400, 1024)], "sketch", 8),
+                                             ([(2716, 2016)] * 5, "dense", 24)])
+def test_product_extent_of_large_launches(shapes, err, rank):
+    """Launches that run from HBM, which were slower with 180 to 290 long CTAs than with three rounds of short ones:
+    about one CTA per SM, or more than fill the device.  At 32 accumulator columns one CTA per SM is resident."""
+    np_cols = 16 if rank <= 16 else 32
+    for mode in (0, 1):
+        products = _products(shapes, mode, err)
+        n, _ = _ctas(products, product_extent(products, _base_extent([p[:2] for p in products]), np_cols, rank))
+        assert n <= 176 or n >= 296 or (np_cols == 32 and n % 148 >= 72), (mode, n)
+
+
+def test_product_extent_of_measured_launches():
+    """Launches whose best extents were measured: small ones split down to K = 128 over idle SMs, a tall one into about
+    one CTA per SM, one round at 32 accumulator columns; those that fill the device at the base extent stay there."""
+    def pick(shapes, mode, err, rank):
+        products = _products(shapes, mode, err)
+        base = _base_extent([p[:2] for p in products])
+        extent = product_extent(products, base, 16 if rank <= 16 else 32, rank)
+        return _ctas(products, extent)[0], extent == base
+    for mode in (0, 1):
+        assert pick([(512, 512)], mode, "sketch", 4)[0] >= 20
+        assert 90 <= pick([(640, 5760)] * 2, mode, "sketch", 32)[0] <= 148
+        assert pick([(640, 5760)] * 2, mode, "sketch", 4)[1]
+        assert pick([(1024, 1024)] * 3 + [(4096, 1024)], mode, "sketch", 8)[1]
+        assert pick([(512, 512)] * 8 + [(2048, 512)] * 4, mode, "dense", 8)[1]
+    assert 120 <= pick([(30528, 1024)], 1, "sketch", 8)[0] <= 160
+    assert product_extent([], 384, 16, 4) == 384
