@@ -210,7 +210,7 @@ def product_extent(products, base: int, np_cols: int, rank: int) -> int:
     return best
 
 
-def decompress_rows(block_ctas, off_rows: int, off_width: int) -> int:
+def decompress_rows(block_ctas, off_rows: int, off_width: int, rank: int = 8) -> int:
     """Matrix rows per unit of the decompress kernels, in {8, 4, 2, 1}.
 
     ``block_ctas(rows)``: CTAs of the block-layout kernel at that many rows.  A unit reads a group's Q rows once for
@@ -219,10 +219,14 @@ def decompress_rows(block_ctas, off_rows: int, off_width: int) -> int:
     two 640 x 5760 at rank 4 45 / 31 / 20 / 17 (360), one of them 24 / 17 / 13 / 13 (180), 4096 x 1024 at rank 8
     35 / 23 / 16 / 17 (192), 1024 x 1024 9.8 / 9.0 / 8.9 / 11 (48), 512 x 1024 8.0 / 7.6 / 8.7 / 11 (24),
     four 64 x 1152 7.7 / 8.1 / 9.3 / 12 (12): eight from two CTAs per SM on, four or two from 96 CTAs on.
+    Above rank 8 the Q rows are most of the traffic and eight rows are the best from 96 CTAs on, although a CTA's 115 KB
+    leave one per SM (16 padded columns): at rank 16 512 x 2048 19 / 15 / 14 / 16 (48), 2048 x 1024 36 / 28 / 25 / 16
+    (96), 512 x 5760 49 / 27 / 25 / 16 (144), 4096 x 1024 64 / 41 / 37 / 31 (192), 2048 x 8192 241 / 143 / 129 / 88 (800);
+    at rank 12 512 x 5760 58 / 36 / 23 / 15, at rank 32 164 / 85 / 49 / 30.
     ``off_rows`` / ``off_width``: rows and widest sketch of the matrices that go to the column-order kernels (dense
     or no error feedback among them: width 0), whose tile is a block of rows with one accumulator row each in shared
     memory: the most that fit while every SM still gets a few CTAs."""
-    for rows, ctas in ((8, 2 * 148), (4, 96), (2, 96)):
+    for rows, ctas in ((8, 2 * 148 if rank <= 8 else 96), (4, 96), (2, 96)):
         if off_rows == 0 and block_ctas(rows) >= ctas:
             return rows
         if off_rows and rows * off_width * 4 <= SMEM_BUDGET // 4 and \
@@ -501,7 +505,7 @@ class PowerSGDEngine(_EngineBase):
         off_rows = sum(e.n for k, e in enumerate(plan.mats) if not on_blocks[k])
         off_W = max((w for k, w in enumerate(self.widths) if not on_blocks[k]), default=0)
         self.d_rows = decompress_rows(lambda rows: sum(math.ceil(units(e, W, rows) / 8) for e, W in on_list),
-                                      off_rows, off_W)
+                                      off_rows, off_W, self.max_rank)
         if os.environ.get("CONEF_D_ROWS"):
             self.d_rows = int(os.environ["CONEF_D_ROWS"])
         self.d_smem = self.d_rows * off_W * 4

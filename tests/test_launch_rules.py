@@ -19,6 +19,13 @@ def test_decompress_rows_of_block_layout_matrices(shapes, rows):
     assert decompress_rows(_block_ctas(shapes), 0, 0) == rows
 
 
+@pytest.mark.parametrize("shapes,rank,rows", [([(4096, 102)], 16, 8), ([(640, 576)], 12, 8), ([(2048, 102)], 16, 8), ([(512, 576)], 32, 8),
+                                              ([(2048, 819)], 16, 8), ([(512, 204)], 16, 4), ([(4096, 102)], 8, 4), ([(640, 576)] * 2, 4, 8)])
+def test_decompress_rows_by_rank(shapes, rank, rows):
+    """Above rank 8 the Q rows of a group are most of what a unit reads: the measured best rows per unit."""
+    assert decompress_rows(_block_ctas(shapes), 0, 0, rank) == rows
+
+
 @pytest.mark.parametrize("off_rows,width,rows", [(3552, 0, 8), (3551, 0, 4), (888, 10, 2), (887, 10, 1), (10_000, 1600, 8),
                                                  (10_000, 1601, 4), (10_000, 12_801, 1), (10_000, 50_000, 1)])
 def test_decompress_rows_of_column_order_matrices(off_rows, width, rows):
