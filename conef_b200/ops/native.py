@@ -218,13 +218,17 @@ _OPTIONAL = {}
 
 
 # How many kernels one call of an entry point enqueues (memsets not counted);
-# everything not listed launches exactly one.  Host-only entry points launch none.
+# everything not listed launches exactly one.  Host-only entry points launch none.  Entry points whose
+# number of launches depends on their arguments are listed with 0 and counted by their callers.
 _KERNELS_PER_CALL = {
-    "conef_lamb_step": 3, "conef_lamb_step_ordered": 3, "conef_lamb_scratch_floats": 0, "conef_orthogonalize_packed": 3, "conef_orthogonalize_fused": 3, "conef_lowrank_correct": 2, "conef_topk_keep": 7, "conef_topk_chunk": 0, "conef_orth_last_launches": 0, "conef_psgd_run": 0, "conef_psgd_plan_size": 0, "conef_mat_size": 0, "conef_randblock_run": 0, "conef_randblock_plan_size": 0, "conef_psgd_step": 0, "conef_psgd_plan_release": 0, "conef_version": 0, "conef_tc_supported": 0, "conef_tc_encode_maps": 0, "conef_last_error": 0,
+    "conef_lamb_step": 3, "conef_lamb_step_ordered": 0, "conef_lamb_scratch_floats": 0, "conef_orthogonalize_packed": 3, "conef_orthogonalize_fused": 3, "conef_lowrank_correct": 2, "conef_topk_keep": 7, "conef_topk_chunk": 0, "conef_orth_last_launches": 0, "conef_psgd_run": 0, "conef_psgd_plan_size": 0, "conef_mat_size": 0, "conef_randblock_run": 0, "conef_randblock_plan_size": 0, "conef_psgd_step": 0, "conef_psgd_plan_release": 0, "conef_version": 0, "conef_tc_supported": 0, "conef_tc_encode_maps": 0, "conef_last_error": 0,
+    "conef_randblock_starts": 0, "conef_sketch3_query_group": 0, "conef_sketch3_update_group": 0,
     "conef_ipc_get_handle": 0, "conef_ipc_open_handle": 0, "conef_ipc_close_handle": 0,
     "conef_cpu_hash_table": 0, "conef_cpu_sketch_query": 0, "conef_cpu_sketch_update": 0,
     "conef_cpu_gram_schmidt": 0,
 }
+RANDBLOCK_STARTS = 256      # block offsets per launch (csrc/blocks.cu:RB_STARTS)
+SKETCH3_GROUP = 32          # matrices per launch (csrc/sketch.cu:SK3_GROUP)
 launch_count = 0  # kernels enqueued through this binding since import (see reset_launch_count)
 
 

@@ -128,3 +128,4 @@ class FusedLAMB(Optimizer):
             tab["scratch"].data_ptr(), float(group["lr"]), float(b1), float(b2), float(group["eps"]), int(step),
             int(bool(group["bias_correction"])), float(self.grad_scale), float(group["max_grad_norm"] or 0.0),
             native.stream_ptr(params[0].device)), "lamb_step")
+        native.launch_count += 3 if (group["max_grad_norm"] or 0.0) > 0 else 2

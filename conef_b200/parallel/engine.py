@@ -969,6 +969,7 @@ class PowerSGDEngine(_EngineBase):
                 copy = torch.empty_like(work)
                 native.check(lib.conef_sketch3_query_group(wp, copy.data_ptr(), group, nm, float(alpha), st),
                              "sketch3_query_group")
+                native.launch_count += math.ceil(nm / native.SKETCH3_GROUP)
             else:
                 for cnt, e in enumerate(plan.mats):
                     comps[cnt].query(work[e.g_off : e.g_off + e.numel], alpha)
@@ -983,6 +984,7 @@ class PowerSGDEngine(_EngineBase):
             if group is not None:
                 native.check(lib.conef_sketch3_update_group(copy.data_ptr(), wp, group, nm, float(beta), st),
                              "sketch3_update_group")
+                native.launch_count += math.ceil(nm / native.SKETCH3_GROUP)
             else:
                 copy.sub_(work)
                 comps = state.error_dict[bidx]
@@ -1292,7 +1294,10 @@ class RandBlockEngine(_EngineBase):
                 starts[k] = int(rng.choice(b.numel))
         if nb:
             native.check(lib.conef_randblock_starts(self.blks_dev.data_ptr(), starts, nb, st), "randblock_starts")
-            native.launch_count += 1
+            # beside what the executor reports: these launches, and the second gather kernel of a bucket whose
+            # tensors are on both layouts of the hash
+            native.launch_count += math.ceil(nb / native.RANDBLOCK_STARTS) + \
+                int(self.ef_mode == native.EF_SKETCH and 0 < self.nblk_tiles < self.n_tiles)
         symm, slot = self.symm, self.step & 1
         fused = self.slots is not None and os.environ.get("CONEF_FUSED", "1") == "1"
         holder = self.slots if fused else symm

@@ -1,5 +1,6 @@
 """Hook-level equivalence on one B200: native engine vs the PyTorch-ops path vs the CPU oracle."""
 import argparse
+import re
 
 import pytest
 import torch
@@ -623,3 +624,44 @@ def test_three_hundred_steps_native_tensorcore_path_converges_like_the_torch_pat
     assert last_n < 0.5 * first_n and last_t < 0.5 * first_n
     assert last_n <= 1.5 * last_t + 0.1 and last_t <= 1.5 * last_n + 0.1
     assert last_n <= 3.0 * last_a + 0.3
+
+
+def _kernels_and_count(fn):
+    """(kernels of this library that ``fn`` enqueued, as the profiler saw them; the binding's launch counter)."""
+    from torch.profiler import ProfilerActivity, profile
+
+    torch.cuda.synchronize()
+    native.reset_launch_count()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    counted = native.reset_launch_count()
+    names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    return [n for n in names if re.match(r"(void )?(\(anonymous namespace\)::)?k_[a-z]", n)], counted
+
+
+@pytest.mark.parametrize("what", ["randomblock", "randomblock_300", "sketch3", "sketch3_40", "lamb", "lamb_clip"])
+def test_launch_counter_matches_the_profiler(single_rank_group, what):
+    """Entry points that take one launch per 256 block offsets or 32 matrices, and LAMB with and without clipping."""
+    many = [(20, 40 + k % 7) for k in range(300 if what.endswith("300") else 40)]
+    if what.startswith("lamb"):
+        from conef_b200.optim import FusedLAMB
+
+        p = torch.nn.Parameter(torch.randn(1000, device=DEV))
+        p.grad = torch.randn(1000, device=DEV)
+        opt = FusedLAMB([p], max_grad_norm=1.0 if what == "lamb_clip" else 0.0)
+        step = opt.step
+    elif what.startswith("randomblock"):
+        state = cb.RandomBlockState(None, start_compression_iter=2, use_error_compression=True, sketch_size=0.5)
+        bucket, hook = FakeBucket(many if "_" in what else SHAPES, device=DEV), cb.RandomBlock_hook
+    else:
+        state = cb.PowerSGDState(None, start_powerSGD_iter=2, matrix_approximation_rank=2, use_error_compression=True,
+                                 error_compressor="count_sketch3", sketch_size=0.5)
+        bucket, hook = FakeBucket(many if "_" in what else SHAPES, device=DEV), cb.powerSGD_hook
+    if not what.startswith("lamb"):
+        state.iter = 2
+        step = lambda: hook(state, bucket).wait()
+    for _ in range(5):
+        step()
+    kernels, counted = _kernels_and_count(step)
+    assert len(kernels) == counted > 0, kernels
