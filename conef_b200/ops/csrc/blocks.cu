@@ -506,12 +506,10 @@ k_randblock_gather_sketch_blk(const ConefBlk* __restrict__ blks, const int2* __r
   conef_publish_if_last(pub, gridDim.x);
 }
 
-// segs / total_unc / staging_unc: the uncompressed tensors (may be empty).  done != NULL with
-// world > 1: the CTA that finishes last stores epoch (+ *epoch_base) into peer_flags[p][rank].
 // New block offsets of a step into the device's block table.  They arrive by value with the launch (RB_STARTS of
 // them at a time): the whole table through a pinned buffer, with a copy and an event per step to know when the
-// buffer was free again, cost the host
-// (with the offset draws) about 40 us per hook call: 137 -> 96 us on the LSTM bucket, 126 -> 92 us on WideResNet's.
+// buffer was free again, cost the host (with the offset draws) about 40 us per hook call: 138 -> 92 us on the LSTM
+// bucket, 127 -> 86 us on WideResNet's.
 constexpr int RB_STARTS = 256;
 struct RbStarts { long long v[RB_STARTS]; };
 __global__ void __launch_bounds__(RB_STARTS)
@@ -531,6 +529,8 @@ extern "C" int conef_randblock_starts(ConefBlk* blks, const long long* starts, i
   return 0;
 }
 
+// segs / total_unc / staging_unc: the uncompressed tensors (may be empty).  done != NULL with
+// world > 1: the CTA that finishes last stores epoch (+ *epoch_base) into peer_flags[p][rank].
 extern "C" int conef_randblock_gather_ex(const ConefBlk* blks, const int2* tiles, int ntiles, int nblk_tiles,
                                          int rows_per_cta, float* bucket, float* staging, float gather_scale, float* sketch,
                                          const int32_t* tables, const int32_t* counts, float* dense_err,

@@ -631,14 +631,18 @@ def test_lowrank_correct_rows_and_ranks(c1, c2):
         assert float((got - w).abs().max()) <= 2e-5 * float(w.abs().max())
 
 
+@pytest.mark.parametrize("form", ["cluster", "one_launch"])
 @pytest.mark.parametrize("r", [1, 2, 3, 4, 5, 8, 11, 16, 17, 32])
-def test_orthogonalize_cluster_every_column_padding(r):
-    """The cluster form at every padding of the column count (1, 2, 4, 8, 16, 32 columns in registers) and at row
-    counts around the cluster's and the warps' shares, against 64 bits.  Tolerance: the Gram-Schmidt of a random
-    block is well conditioned; two rounds of 32-bit sums stay below 1e-4."""
+def test_orthogonalize_cluster_every_column_padding(r, form):
+    """Both one-launch forms at every column count the kernels are built for (4, 8, 16 and 32) and counts below them,
+    and at row counts around the cluster's, the chunks' and the warps' shares; the barrier form also with a block of
+    60 chunks, so that every group of threads adds up several partials.  Against 64 bits.  Tolerance: the Gram-Schmidt
+    of a random block is well conditioned; two rounds of 32-bit sums stay below 1e-4."""
     gen = torch.Generator().manual_seed(r)
-    blocks = [torch.randn(n, r, generator=gen) for n in (max(r, 1), r + 7, 64 + r, 513, 2049, 8192)]
-    for i, (b, q) in enumerate(zip(blocks, _orth_on_device([b.clone() for b in blocks], cluster=True))):
+    rows = (max(r, 1), r + 7, 64 + r, 513, 2049, 8192 if form == "cluster" else 30528)
+    blocks = [torch.randn(n, r, generator=gen) for n in rows]
+    got = _orth_on_device([b.clone() for b in blocks], cluster=form == "cluster", one_launch=form == "one_launch")
+    for i, (b, q) in enumerate(zip(blocks, got)):
         if i == 0 and r > 1:      # square: the last column's direction is what is left over, badly conditioned
             assert torch.isfinite(q).all()
             continue
