@@ -182,9 +182,9 @@ def product_time(groups, extent: int, np_cols: int, rank: int) -> float:
 def product_extent(products, base: int, np_cols: int, rank: int) -> int:
     """K extent of the CTAs of one tensor-core launch over ``products``: (output rows, K, output, atomic).
 
-    ``base`` (three rounds of CTAs of K = 384 to 1,024) unless another extent is at least 14 % shorter by
-    ``product_time``: with that margin two of those 147 launches were slower than at ``base`` (by 3 and 4 %), with
-    10 % nine were, by up to 15 %.  Measured in us, P and Q, base -> choice: 512 x 512 at rank 4 8.4, 8.4 -> 4.9, 5.0;
+    ``base`` (three rounds of CTAs of K = 384 to 1,024) unless another extent is at least 13 % shorter by
+    ``product_time``.  Over 233 launches, whole-model buckets among them, the product then takes 11 % less time than at
+    ``base`` on average and two took more (3 and 4 %); with a margin of 5 % a tenth did.  Measured in us, P and Q, base -> choice: 512 x 512 at rank 4 8.4, 8.4 -> 4.9, 5.0;
     30528 x 1024 at rank 8 33, 42 -> 29, 26, at rank 24 61, 66 -> 41, 30; two 640 x 5760 at rank 32 22, 21 -> 14, 12;
     38400 x 1024 40, 46 -> 38, 31; five 2716 x 2016 with dense feedback 45, 44 -> 46, 41, at rank 24 70, 70 -> 56, 58."""
     if not products:
@@ -205,7 +205,7 @@ def product_extent(products, base: int, np_cols: int, rank: int) -> int:
             candidates.append(extent)
             last = extent
     best = min((e for e in candidates if e), key=lambda e: product_time(groups, e, np_cols, rank))
-    if product_time(groups, base, np_cols, rank) <= 1.16 * product_time(groups, best, np_cols, rank):
+    if product_time(groups, base, np_cols, rank) <= 1.15 * product_time(groups, best, np_cols, rank):
         return base
     return best
 
