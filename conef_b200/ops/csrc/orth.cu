@@ -316,10 +316,32 @@ constexpr long long ORTH_BARRIER_LIMIT = 2LL * 1000 * 1000;
 // division and one shuffle.  Reading G and R back from shared memory in loops over r took 6,500 cycles per call
 // at r = 8 and 3,000 at r = 4, more than half of the kernel, which went from 22 to 17 us per launch on a
 // BERT-large bucket of 29 MB (r = 8; with the Gram and store loops below).
+// Above eight columns the unrolled elimination costs more than it saves: its registers leave one CTA per SM, so that
+// a launch of more than 18 blocks runs in several rounds, and its code (500 shuffles at 32 columns) is fetched for one
+// pass of one warp.  There the loops over shared memory stay.  us per launch, loops against unrolled: 12 blocks of
+// 512 rows 31 / 33 (r = 16), 64 / 85 (r = 32); 48 blocks 33 / 120 and 72 / 325.
 template <int RP>
 __device__ __forceinline__ void chol_factor(const float (*G)[RP + 1], float (*R)[RP + 1], float* rd, int r,
                                             float shift, float eps) {
   const int lane = threadIdx.x;
+  if (RP > 8) {
+    for (int j = 0; j < r; ++j) {
+      float d = G[j][j];
+      for (int k = 0; k < j; ++k) d = fmaf(-R[k][j], R[k][j], d);
+      const bool dead = !(G[j][j] > 0.f);
+      const float floor_d = shift * G[j][j];
+      if (!(d > floor_d)) d = floor_d;
+      const float rjj = dead ? 0.f : sqrtf(d);
+      if (lane == j) { R[j][j] = rjj; rd[j] = dead ? 0.f : 1.f / (rjj + eps); }
+      if (lane > j && lane < r) {
+        float v = G[j][lane];
+        for (int k = 0; k < j; ++k) v = fmaf(-R[k][j], R[k][lane], v);
+        R[j][lane] = dead ? 0.f : v / rjj;
+      }
+      __syncwarp();
+    }
+    return;
+  }
   float g[RP];                                   // g[k] = G[k][lane], of which k <= lane is used
 #pragma unroll
   for (int k = 0; k < RP; ++k) g[k] = (lane < r && k <= lane) ? G[k][lane] : 0.f;
@@ -403,12 +425,11 @@ __device__ __forceinline__ void gram_partial(const float* xs, int rows, int r,
       out[threadIdx.x] = sum;
     }
   } else {
-    for (int pr = threadIdx.x; pr < PAIRS; pr += OC_THREADS) {
-      const int ca = pr / RP, cb = pr % RP;
+    for (int pr = threadIdx.x; pr < r * r; pr += OC_THREADS) {
+      const int ca = pr / r, cb = pr - ca * r;
       float acc = 0.f;
-      if (ca < r && cb < r)
-        for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
-      out[pr] = acc;
+      for (int i = 0; i < rows; ++i) acc = fmaf(xs[i * S + ca], xs[i * S + cb], acc);
+      out[ca * RP + cb] = acc;
     }
   }
 }
@@ -565,6 +586,7 @@ k_orth_one(const ConefMat* __restrict__ mats, const int2* __restrict__ tiles, in
     __syncthreads();
     // ---- apply: every thread its rows ----
     for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
+      if (RP > 8) asm volatile("" ::: "memory");      // R stays in shared memory: in registers it costs occupancy
       float av[RP], yv[RP];
 #pragma unroll
       for (int k = 0; k < RP; ++k) av[k] = xs[i * S + k];
@@ -630,8 +652,11 @@ __device__ __forceinline__ float ld_dsmem_f32(const float* local_smem, uint32_t 
   return v;
 }
 
+// The second launch bound keeps enough CTAs on an SM for 92, 74, 74 and 55 blocks at once (the factorisation leaves
+// most of an SM idle, so another round costs as much as the first): us for 80 blocks of 512 rows with the bounds and
+// without, 13 / 19 at r = 4, 60 / 179 at r = 16, 134 / 486 at r = 32.
 template <int RP>
-__global__ void __launch_bounds__(OC_THREADS)
+__global__ void __launch_bounds__(OC_THREADS, RP <= 4 ? 5 : RP <= 16 ? 4 : 3)
 k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list, int nmat, int which,
                float* __restrict__ buf, const float* const* __restrict__ peer_bufs,
                const uint32_t* __restrict__ flags, int world, uint32_t epoch, int* __restrict__ status,
@@ -766,6 +791,7 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
     __syncthreads();
     // ---- apply: every thread its rows ----
     for (int i = threadIdx.x; i < rows; i += OC_THREADS) {
+      if (RP > 8) asm volatile("" ::: "memory");      // R stays in shared memory: in registers it costs occupancy
       float av[RP], yv[RP];
 #pragma unroll
       for (int k = 0; k < RP; ++k) av[k] = xs[i * S + k];

@@ -144,3 +144,25 @@ def test_product_extent_of_measured_launches():
         assert pick([(512, 512)] * 8 + [(2048, 512)] * 4, mode, "dense", 8)[1]
     assert 120 <= pick([(30528, 1024)], 1, "sketch", 8)[0] <= 160
     assert product_extent([], 384, 16, 4) == 384
+
+
+def test_gram_schmidt_kernels_keep_their_occupancy(tmp_path):
+    """Registers of the one-launch Gram-Schmidt kernels as the compiler reports them: a bucket of some dozens of
+    matrices runs in one round only while enough thread-block clusters of eight 256-thread CTAs fit on the device."""
+    import re
+    import subprocess
+
+    from conef_b200.ops import build
+
+    try:
+        nvcc = build.find_nvcc()
+    except RuntimeError:
+        pytest.skip("nvcc not found")
+    cmd = [nvcc, *build.NVCC_FLAGS, "-Xptxas", "-v", "-I", str(build.CSRC), "-c", str(build.CSRC / "orth.cu"), "-o",
+           str(tmp_path / "orth.o")]
+    out = subprocess.run(cmd, capture_output=True, text=True, check=True).stderr
+    regs = {(m[1], int(m[2])): int(m[3]) for m in
+            re.finditer(r"properties for _Z\d+(k_orth_\w+?)ILi(\d+)E.*?Used (\d+) registers", out, re.S)}
+    per_sm = lambda r: 65536 // (256 * ((r + 7) // 8 * 8))
+    assert [per_sm(regs["k_orth_cluster", rp]) >= n for rp, n in ((4, 5), (8, 4), (16, 4), (32, 3))] == [True] * 4, regs
+    assert all(per_sm(regs["k_orth_one", rp]) >= 2 for rp in (4, 8, 16, 32)), regs
