@@ -144,11 +144,12 @@ def product_time(groups, extent: int, np_cols: int, rank: int) -> float:
     ``groups``: {products that add into one output: how many such outputs}, a product being (output rows, K, whether
     it adds with atomics even when one CTA covers K).  A CTA costs a fixed time (prologue, drain; more per output
     column with atomics) and, per unit of K, what a lone CTA reaches or its share of the bandwidth.  From L2, rounds of
-    CTAs follow each other and the last one shares the bandwidth among fewer.  From HBM the bandwidth decides, which
-    is best with about one CTA per SM (30528 x 1024, Q: 135 CTAs 26 us, 180 27, 216 to 297 29 to 34; six 4390 x 1216
-    with dense feedback, Q: 120 CTAs 27 us, 240 33).  CTAs that split one output add to the same addresses, one after
-    another.  Fitted to 147 launches at up to 20 extents each (64 x 576 to 38400 x 1024, ranks 1 to 32, with and
-    without error records), of which a third ran from HBM: the pick is on average 2 % slower than the best measured."""
+    CTAs follow each other and the last one shares the bandwidth among fewer.  From HBM the bandwidth decides, and a
+    launch of more CTAs than are resident gets less of it: 30528 x 1024 at rank 8, Q: 135 to 288 CTAs 25 to 27 us, 360
+    to 720 32 to 40; seven 1536 x 2048 with dense feedback, Q: 224 CTAs 30 us, 448 33, 896 37.  CTAs that split one
+    output add to the same addresses, one after another.  Fitted to launches inside hook calls at up to 17 extents each
+    (64 x 576 to 30528 x 1024, ranks 1 to 32, with and without error records): over 246 of them the pick is on average
+    2 % slower than the best extent measured and 11 % faster than ``base`` of product_extent."""
     slots = product_slots(np_cols)
     n = work = longest = adds = most = nbytes = 0
     for group, count in groups.items():
@@ -165,11 +166,11 @@ def product_time(groups, extent: int, np_cols: int, rank: int) -> float:
         most = max(most, adders)
     columns, mean = rank * adds / n, work / n
     if nbytes > LARGE_LAUNCH:
-        fixed = 1.1 + 0.22 * columns
-        crowd = 0.15 * min(1.0, max(0.0, (n - 148) / 35)) if slots > 148 else 0.0
-        t = max(fixed * max(1.0, n / slots) + nbytes / 6.9e6 * (1 + crowd), fixed + 0.0105 * longest)
+        fixed = 2.0 + 0.18 * columns
+        t = fixed * max(1.0, n / slots) + nbytes / (8.6e6 if n <= slots or slots == 148 else 6.6e6)
+        t = max(t, fixed + 0.012 * longest)
         if slots == 148:
-            t = max(t, math.ceil(n / slots) * (fixed + 0.009 * mean))
+            t = max(t, math.ceil(n / slots) * (fixed + 0.012 * mean))
     else:
         fixed = 4.0 + 0.09 * columns
         per_k = lambda ctas: max(0.0088, 3.4e-5 * ctas)
@@ -182,11 +183,10 @@ def product_time(groups, extent: int, np_cols: int, rank: int) -> float:
 def product_extent(products, base: int, np_cols: int, rank: int) -> int:
     """K extent of the CTAs of one tensor-core launch over ``products``: (output rows, K, output, atomic).
 
-    ``base`` (three rounds of CTAs of K = 384 to 1,024) unless another extent is at least 13 % shorter by
-    ``product_time``.  Over 233 launches, whole-model buckets among them, the product then takes 11 % less time than at
-    ``base`` on average and two took more (3 and 4 %); with a margin of 5 % a tenth did.  Measured in us, P and Q, base -> choice: 512 x 512 at rank 4 8.4, 8.4 -> 4.9, 5.0;
-    30528 x 1024 at rank 8 33, 42 -> 29, 26, at rank 24 61, 66 -> 41, 30; two 640 x 5760 at rank 32 22, 21 -> 14, 12;
-    38400 x 1024 40, 46 -> 38, 31; five 2716 x 2016 with dense feedback 45, 44 -> 46, 41, at rank 24 70, 70 -> 56, 58."""
+    ``base`` (three rounds of CTAs of K = 384 to 1,024) unless another extent is at least 9 % shorter by
+    ``product_time``.  Measured inside hook calls in us, P and Q, base -> choice: 512 x 512 at rank 4 8.0, 7.8 -> 4.8,
+    5.0; 30528 x 1024 at rank 8 39, 40 -> 31, 26, at rank 24 65, 70 -> 46, 41; two 640 x 5760 at rank 32 22, 21 -> 15, 13;
+    with dense feedback seven 1536 x 2048 at rank 4 40, 38 -> 39, 30, six 1024 x 4096 at rank 16 53, 48 -> 46, 42."""
     if not products:
         return base
     outputs = {}
@@ -205,7 +205,7 @@ def product_extent(products, base: int, np_cols: int, rank: int) -> int:
             candidates.append(extent)
             last = extent
     best = min((e for e in candidates if e), key=lambda e: product_time(groups, e, np_cols, rank))
-    if product_time(groups, base, np_cols, rank) <= 1.15 * product_time(groups, best, np_cols, rank):
+    if product_time(groups, base, np_cols, rank) <= 1.1 * product_time(groups, best, np_cols, rank):
         return base
     return best
 
