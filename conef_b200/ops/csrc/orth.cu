@@ -652,11 +652,12 @@ __device__ __forceinline__ float ld_dsmem_f32(const float* local_smem, uint32_t 
   return v;
 }
 
-// The second launch bound keeps enough CTAs on an SM for 92, 74, 74 and 55 blocks at once (the factorisation leaves
-// most of an SM idle, so another round costs as much as the first): us for 80 blocks of 512 rows with the bounds and
-// without, 13 / 19 at r = 4, 60 / 179 at r = 16, 134 / 486 at r = 32.
-template <int RP>
-__global__ void __launch_bounds__(OC_THREADS, RP <= 4 ? 5 : RP <= 16 ? 4 : 3)
+// PER_SM: CTAs that must fit on an SM.  The factorisation leaves most of an SM idle, so another round costs as much as
+// the first: us for 80 blocks of 512 rows with and without the bound 13 / 19 at r = 4, 60 / 179 at r = 16, 134 / 486 at
+// r = 32.  Up to eight columns one CTA less per SM has registers to spare (12 blocks of 512 rows at r = 8 15.0 us
+// against 15.7, 4 of 2,048 17.4 against 18.9) and is taken for the blocks that still make one round.
+template <int RP, int PER_SM>
+__global__ void __launch_bounds__(OC_THREADS, PER_SM)
 k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list, int nmat, int which,
                float* __restrict__ buf, const float* const* __restrict__ peer_bufs,
                const uint32_t* __restrict__ flags, int world, uint32_t epoch, int* __restrict__ status,
@@ -832,7 +833,7 @@ k_orth_cluster(const ConefMat* __restrict__ mats, const int2* __restrict__ list,
 
 // *launched: false when the rows of the largest block do not fit in shared memory or the device cannot
 // hold one cluster; the caller then takes another form.
-template <int RP>
+template <int RP, int PER_SM>
 static int launch_orth_cluster(const ConefMat* mats, const int2* list, int nmat, int max_rows, int seg_ctas, int which,
                                float* buf, float eps, const float* const* peer_bufs, const uint32_t* flags, int world,
                                uint32_t epoch, int* status, long long spin_limit, float* packed, int packed_np,
@@ -850,7 +851,7 @@ static int launch_orth_cluster(const ConefMat* mats, const int2* list, int nmat,
   CONEF_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return 0;
   if (smem > configured[dev]) {      // static + dynamic shared memory may pass 48 KB well before the dynamic part does
-    CONEF_CUDA(cudaFuncSetAttribute(k_orth_cluster<RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CONEF_CUDA(cudaFuncSetAttribute(k_orth_cluster<RP, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev] = smem;
   }
   cudaLaunchConfig_t cfg;
@@ -871,12 +872,12 @@ static int launch_orth_cluster(const ConefMat* mats, const int2* list, int nmat,
   if (cluster_ok[dev] == 0 || smem > probed[dev]) {
     probed[dev] = smem;
     int nclusters = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, k_orth_cluster<RP>, &cfg);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, k_orth_cluster<RP, PER_SM>, &cfg);
     cluster_ok[dev] = (e == cudaSuccess && nclusters > 0) ? 1 : -1;
     if (e != cudaSuccess) (void)cudaGetLastError();
   }
   if (cluster_ok[dev] < 0) return 0;
-  CONEF_CUDA(cudaLaunchKernelEx(&cfg, k_orth_cluster<RP>, mats, list, nmat, which, buf, peer_bufs, flags, world, epoch,
+  CONEF_CUDA(cudaLaunchKernelEx(&cfg, k_orth_cluster<RP, PER_SM>, mats, list, nmat, which, buf, peer_bufs, flags, world, epoch,
                                 status, spin_limit, epoch_base, eps, packed, packed_np, X));
   *launched = true;
   return 0;
@@ -936,14 +937,16 @@ extern "C" int conef_orthogonalize_fused(const ConefMat* mats, const int2* tiles
     // one cluster per block when a CTA's share of the largest block fits in shared memory
     bool launched = false;
     int rc;
-#define CONEF_ORTH_CL(RP)                                                                                        \
-    rc = launch_orth_cluster<RP>(mats, X.cl_list, X.cl_nmat, X.cl_max_rows, seg_ctas, which, buf, eps, peer_bufs, \
+#define CONEF_ORTH_CL(RP, PER_SM)                                                                                \
+    rc = launch_orth_cluster<RP, PER_SM>(mats, X.cl_list, X.cl_nmat, X.cl_max_rows, seg_ctas, which, buf, eps, peer_bufs, \
                                  flags, world, epoch, status, spin_limit, packed, packed_np, epoch_base, X, stream, \
                                  &launched)
-    if (X.max_rank <= 4) CONEF_ORTH_CL(4);
-    else if (X.max_rank <= 8) CONEF_ORTH_CL(8);
-    else if (X.max_rank <= 16) CONEF_ORTH_CL(16);
-    else CONEF_ORTH_CL(32);
+    // blocks of one round: per GPC of 16 to 18 SMs, PER_SM of its CTAs on each, in clusters of eight
+    const int blocks = X.cl_nmat + (seg_ctas + OCL - 1) / OCL;
+    if (X.max_rank <= 4) { if (blocks <= 64) CONEF_ORTH_CL(4, 4); else CONEF_ORTH_CL(4, 5); }
+    else if (X.max_rank <= 8) { if (blocks <= 48) CONEF_ORTH_CL(8, 3); else CONEF_ORTH_CL(8, 4); }
+    else if (X.max_rank <= 16) CONEF_ORTH_CL(16, 4);
+    else CONEF_ORTH_CL(32, 3);
 #undef CONEF_ORTH_CL
     if (rc != 0) return rc;
     if (launched) { g_orth_launches = 1; return 0; }

@@ -167,8 +167,11 @@ def test_gram_schmidt_kernels_keep_their_occupancy(tmp_path):
     cmd = [nvcc, *build.NVCC_FLAGS, "-Xptxas", "-v", "-I", str(build.CSRC), "-c", str(build.CSRC / "orth.cu"), "-o",
            str(tmp_path / "orth.o")]
     out = subprocess.run(cmd, capture_output=True, text=True, check=True).stderr
-    regs = {(m[1], int(m[2])): int(m[3]) for m in
-            re.finditer(r"properties for _Z\d+(k_orth_\w+?)ILi(\d+)E.*?Used (\d+) registers", out, re.S)}
     per_sm = lambda r: 65536 // (256 * ((r + 7) // 8 * 8))
-    assert [per_sm(regs["k_orth_cluster", rp]) >= n for rp, n in ((4, 5), (8, 4), (16, 4), (32, 3))] == [True] * 4, regs
-    assert all(per_sm(regs["k_orth_one", rp]) >= 2 for rp in (4, 8, 16, 32)), regs
+    found = {}
+    for m in re.finditer(r"properties for _Z\d+(k_orth_\w+?)ILi(\d+)E\w*?v?P.*?Used (\d+) registers", out, re.S):
+        found.setdefault((m[1], int(m[2])), []).append(per_sm(int(m[3])))
+    for columns, most, least in ((4, 5, 4), (8, 4, 3), (16, 4, 4), (32, 3, 3)):      # many blocks, and the fewer form
+        got = found["k_orth_cluster", columns]
+        assert max(got) >= most and min(got) >= least, found
+        assert min(found["k_orth_one", columns]) >= 2, found
