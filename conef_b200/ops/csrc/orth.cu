@@ -4,7 +4,7 @@
 // per column per matrix (communication/powerSGD_hook.py:12-43).  A tall block (30,528 x 8 for
 // BERT's embedding) must not be walked by one CTA, so Gram-Schmidt is done through the Gram
 // matrix, which needs only row-parallel passes:
-//   k_gram      : G = A^T A, one CTA per (matrix, chunk of rows), partial sums by atomics.
+//   k_gram      : G = A^T A, one CTA per (matrix, chunk of rows), a partial sum per chunk.
 //                 With world > 1 the chunk first sums the peers' copies of its rows
 //                 (all-reduce over NVLink peer loads fused into the pass, bounded flag wait).
 //   k_qr_apply  : every CTA factors G = R^T R (r <= 32: a warp does it in shared memory),
